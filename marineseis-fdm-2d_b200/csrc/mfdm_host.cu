@@ -1490,7 +1490,7 @@ int adjoint_build(mfdm_model* m) {
   Coef C = m->C;
   C.srcx = -1;  // the operator without the source
   C.src_pos = nullptr;
-  const int stage = 1;  // a middle stage: out = U^n + c k, with U^n = 0
+  const int stage = 2;  // the third stage: out = U^n + c k, with U^n = 0, and no accumulator
   const float cc = C.rk_c[stage], scale = 1.0f / cc;
   mfdm::StageMaps maps;
   maps.fin = m->fst[1]; maps.sin = m->sst[1];

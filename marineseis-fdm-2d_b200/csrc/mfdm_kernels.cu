@@ -24,8 +24,8 @@
 // segment down in chunks of kR rows with 3-D TMA boxes (cp.async.bulk.tensor)
 // completing on the chunk slot's mbarrier: all stencil fields of the stage
 // input with a 4-column halo into a row-contiguous ring (kNS chunk
-// slots), and the point-wise inputs (coefficients, U^n, accumulator) into the
-// slot's point-wise buffer.
+// slots), and the point-wise inputs (coefficients, and U^n or the
+// accumulator) into the slot's point-wise buffer.
 // Warps 0-7 compute one cell each per chunk purely from shared memory and
 // store the stage output and accumulator straight to HBM, coalesced along x.
 // Each field row thus crosses HBM once per stage; only the 3-row halo above
@@ -77,10 +77,10 @@ static_assert(kNS >= 3 && kNP >= 1, "ring depths");
 static_assert(2 * (kNS + kNP) * 8 <= kBarBytes, "barrier region too small");
 
 // Point-wise inputs staged per chunk, by stage kind: coefficients, then U^n
-// (middle stages), then the accumulator (middle and last stages).
+// (second and third stage) or the accumulator (last stage).
 template <int NST, int NCOEF, int KIND>
 struct PW {
-  static constexpr int n = NCOEF + (KIND == kStageMid ? 2 * NST : (KIND == kStageLast ? NST : 0));
+  static constexpr int n = NCOEF + (KIND == kStageFirst ? 0 : NST);
 };
 
 // Shared memory of one segment block: barriers, the stencil ring of kRingRows
@@ -137,7 +137,7 @@ struct Bars {
 // previous chunk is released: one 3-D TMA box with all stencil fields of kR
 // rows and the column halo (chunks of the first and last slot a second time,
 // past the ring's other end). The point-wise inputs of chunk j (j = 0 .. nch-1:
-// coefficients, U^n, accumulator, up to three boxes) go to point-wise slot
+// coefficients, then U^n or the accumulator) go to point-wise slot
 // j % kNP once chunk j - kNP is computed, and are issued right after stencil
 // chunk j + D, D = kNS - 1 - kNP: the two waits then become due together, so
 // neither ring holds up the other.
@@ -161,12 +161,9 @@ __device__ __forceinline__ void produce(const Segment& sg, const CUtensorMap* in
     float* d = slots + ps * NPW * kF;
     mbar_arrive_expect_tx(&B.pfull[ps], kPwBytes);
     tma_load_3d(d, coef_map, sg.x0, q0, 0, &B.pfull[ps]);
-    if (KIND == kStageMid) {
-      tma_load_4d(d + NCOEF * kF, un_map, sg.x0, q0, 0, shot, &B.pfull[ps]);
-      tma_load_4d(d + (NCOEF + NST) * kF, acc_map, sg.x0, q0, 0, shot, &B.pfull[ps]);
-    } else if (KIND == kStageLast) {
-      tma_load_4d(d + NCOEF * kF, acc_map, sg.x0, q0, 0, shot, &B.pfull[ps]);
-    }
+    if (KIND != kStageFirst)
+      tma_load_4d(d + NCOEF * kF, KIND == kStageLast ? acc_map : un_map, sg.x0, q0, 0, shot,
+                  &B.pfull[ps]);
     return true;
   };
   for (int k = -1; k <= sg.nch; ++k) {
@@ -317,15 +314,15 @@ __device__ __forceinline__ void fluid_segment(const Coef& C, const Fields& in, c
     float* const accs[3] = {acc.fvx, acc.fvz, acc.fp};
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
+      const float y = A.at(f, 0, 0);
       if (KIND == kStageFirst) {
-        const float u0 = A.at(f, 0, 0);
-        outs[f][i] = fmaf(cc, kv[f], u0);
-        accs[f][i] = fmaf(w, kv[f], u0);
-      } else if (KIND == kStageMid) {
-        outs[f][i] = fmaf(cc, kv[f], pw[(NCOEF + f) * F]);
-        accs[f][i] = fmaf(w, kv[f], pw[(NCOEF + NST + f) * F]);
+        outs[f][i] = fmaf(cc, kv[f], y);
+      } else if (KIND == kStageLast) {
+        outs[f][i] = rk_last(kv[f], y, pw[(NCOEF + f) * F], cc);
       } else {
-        outs[f][i] = fmaf(cc, kv[f], pw[(NCOEF + f) * F]);
+        const float u0 = pw[(NCOEF + f) * F];
+        outs[f][i] = fmaf(cc, kv[f], u0);
+        if (KIND == kStageSecond) accs[f][i] = rk_acc(kv[f], y, u0, w);
       }
     }
     if (sd) {
@@ -411,15 +408,15 @@ __device__ __forceinline__ void solid_segment(const Coef& C, const Fields& in, c
     float* const accs[5] = {acc.svx, acc.svz, acc.ssx, acc.ssz, acc.ssxz};
 #pragma unroll
     for (int f = 0; f < 5; ++f) {
+      const float y = A.at(f, 0, 0);
       if (KIND == kStageFirst) {
-        const float u0 = A.at(f, 0, 0);
-        outs[f][i] = fmaf(cc, kv[f], u0);
-        accs[f][i] = fmaf(w, kv[f], u0);
-      } else if (KIND == kStageMid) {
-        outs[f][i] = fmaf(cc, kv[f], pw[(NCOEF + f) * F]);
-        accs[f][i] = fmaf(w, kv[f], pw[(NCOEF + NST + f) * F]);
+        outs[f][i] = fmaf(cc, kv[f], y);
+      } else if (KIND == kStageLast) {
+        outs[f][i] = rk_last(kv[f], y, pw[(NCOEF + f) * F], cc);
       } else {
-        outs[f][i] = fmaf(cc, kv[f], pw[(NCOEF + f) * F]);
+        const float u0 = pw[(NCOEF + f) * F];
+        outs[f][i] = fmaf(cc, kv[f], u0);
+        if (KIND == kStageSecond) accs[f][i] = rk_acc(kv[f], y, u0, w);
       }
     }
     if (sd) {
@@ -503,7 +500,7 @@ __device__ __forceinline__ void interface_strip(const Coef& C, const Fields& in,
   for (int f = 0; f < 8; ++f) {
     const size_t i = f < 3 ? fi : si;
     if (KIND == kStageLast) {
-      C.ipre[(size_t)f * P + ix] = fmaf(c, kv[f], accs[f][i]);
+      C.ipre[(size_t)f * P + ix] = rk_last(kv[f], uin[f], accs[f][i], c);
     } else {
       rk_update<KIND>(kv[f], uin[f], uns[f], outs[f], accs[f], i, c, w);
     }
@@ -533,7 +530,7 @@ __device__ __forceinline__ void interface_strip(const Coef& C, const Fields& in,
 }
 
 // One RK stage: `s` indexes the Ricker table; cc and w are the stage's RK
-// weights (out = base + cc k, accumulator += w k).
+// weights (rk_update in mfdm_device.cuh).
 template <int DIR, int KIND, bool CPML>
 __global__ void __launch_bounds__(kThreads, MFDM_MIN_BLOCKS)
     stage_kernel(Coef C0, Fields in0, Fields out0, Fields un0, Fields acc0,
@@ -566,7 +563,7 @@ static size_t smem_for_kind() {
   return f > so ? f : so;
 }
 
-size_t smem_bytes() { return smem_for_kind<kStageMid>(); }
+size_t smem_bytes() { return smem_for_kind<kStageSecond>(); }
 
 static int seg_rows_of(const Coef& C) { return C.seg > 0 ? C.seg : default_seg_rows(C); }
 
@@ -585,7 +582,7 @@ static cudaError_t launch_one(const Coef& C, const Fields& in, const Fields& out
   int ntx, nbf, nbs, nbi;
   const int seg = seg_rows_of(C), nshots = C.nshots > 0 ? C.nshots : 1;
   grid_of(C.nx, C.nzf, C.nzs, seg, &ntx, &nbf, &nbs, &nbi);
-  const float cc = C.rk_c[s], w = (KIND == kStageLast) ? 0.f : C.rk_w[s];
+  const float cc = C.rk_c[s], w = (KIND == kStageSecond) ? C.rk_w[s] : 0.f;
   const unsigned grid = unsigned(nbi + nbf + nbs) * unsigned(nshots);
   stage_kernel<DIR, KIND, CPML><<<grid, kThreads, smem_for_kind<KIND>(), st>>>(
       C, in, out, un, acc, maps, s, cc, w, ntx, nbi, nbf, nbs, seg, nshots);
@@ -605,10 +602,12 @@ static cudaError_t configure_one() {
 cudaError_t configure() {
   cudaError_t e;
   if ((e = configure_one<kDirF, kStageFirst>()) != cudaSuccess) return e;
-  if ((e = configure_one<kDirF, kStageMid>()) != cudaSuccess) return e;
+  if ((e = configure_one<kDirF, kStageSecond>()) != cudaSuccess) return e;
+  if ((e = configure_one<kDirF, kStageThird>()) != cudaSuccess) return e;
   if ((e = configure_one<kDirF, kStageLast>()) != cudaSuccess) return e;
   if ((e = configure_one<kDirB, kStageFirst>()) != cudaSuccess) return e;
-  if ((e = configure_one<kDirB, kStageMid>()) != cudaSuccess) return e;
+  if ((e = configure_one<kDirB, kStageSecond>()) != cudaSuccess) return e;
+  if ((e = configure_one<kDirB, kStageThird>()) != cudaSuccess) return e;
   return configure_one<kDirB, kStageLast>();
 }
 
@@ -616,14 +615,16 @@ template <bool CPML>
 static cudaError_t launch_stage_bc(const Coef& C, const Fields& in, const Fields& out,
                                   const Fields& un, const Fields& acc, const StageMaps& maps,
                                   int stage, int dir, cudaStream_t st) {
-  const int kind = stage == 0 ? kStageFirst : (stage == 3 ? kStageLast : kStageMid);
+  const int kind = stage;  // kStageFirst .. kStageLast
   if (dir == kDirF) {
     if (kind == kStageFirst) return launch_one<kDirF, kStageFirst, CPML>(C, in, out, un, acc, maps, stage, st);
-    if (kind == kStageMid) return launch_one<kDirF, kStageMid, CPML>(C, in, out, un, acc, maps, stage, st);
+    if (kind == kStageSecond) return launch_one<kDirF, kStageSecond, CPML>(C, in, out, un, acc, maps, stage, st);
+    if (kind == kStageThird) return launch_one<kDirF, kStageThird, CPML>(C, in, out, un, acc, maps, stage, st);
     return launch_one<kDirF, kStageLast, CPML>(C, in, out, un, acc, maps, stage, st);
   }
   if (kind == kStageFirst) return launch_one<kDirB, kStageFirst, CPML>(C, in, out, un, acc, maps, stage, st);
-  if (kind == kStageMid) return launch_one<kDirB, kStageMid, CPML>(C, in, out, un, acc, maps, stage, st);
+  if (kind == kStageSecond) return launch_one<kDirB, kStageSecond, CPML>(C, in, out, un, acc, maps, stage, st);
+  if (kind == kStageThird) return launch_one<kDirB, kStageThird, CPML>(C, in, out, un, acc, maps, stage, st);
   return launch_one<kDirB, kStageLast, CPML>(C, in, out, un, acc, maps, stage, st);
 }
 
@@ -650,7 +651,7 @@ cudaError_t upload_constants_v(const float* srcw25, const float* w7) {
 // per thread at the default 16). A block stages the stage-input fields of its cells with their 3-row,
 // 4-column halo in shared memory with independent float4 loads (zero outside
 // the arrays, as the tensor maps of the ring builds fill), while every thread
-// already has the point-wise operands of its first row in flight: U^n, the
+// already has the point-wise operands of its first row in flight: U^n or the
 // accumulator and the coefficient block's values (metric copies, 1/rho and K
 // or the stiffnesses). 32 warps per SM, no producer warp, no ring barriers.
 // The interface strip is the ring builds' (global loads).
@@ -696,7 +697,7 @@ struct SolidTile : TileAcc<5> {
 // knows, which would otherwise order each field's loads after the previous
 // field's stores).
 template <int NST, int NCOEF>
-struct TilePt { float u[NST], a[NST], k[NCOEF]; };
+struct TilePt { float u[NST], k[NCOEF]; };  // u: U^n, or the accumulator (last stage)
 
 template <int NST, int NCOEF, int KIND>
 __device__ __forceinline__ void tile_load_pt(TilePt<NST, NCOEF>& p, const float* const* un,
@@ -704,8 +705,8 @@ __device__ __forceinline__ void tile_load_pt(TilePt<NST, NCOEF>& p, const float*
                                              size_t nblk, size_t i) {
 #pragma unroll
   for (int f = 0; f < NST; ++f) {
-    if (KIND == kStageMid) p.u[f] = __ldg(un[f] + i);
-    if (KIND != kStageFirst) p.a[f] = acc[f][i];
+    if (KIND == kStageSecond || KIND == kStageThird) p.u[f] = __ldg(un[f] + i);
+    if (KIND == kStageLast) p.u[f] = acc[f][i];
   }
 #pragma unroll
   for (int q = 0; q < NCOEF; ++q) p.k[q] = __ldg(coef + q * nblk + i);
@@ -788,15 +789,14 @@ __device__ __forceinline__ void fluid_tile(const Coef& C, const Fields& in, cons
     float* const accs[3] = {acc.fvx, acc.fvz, acc.fp};
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
+      const float y = A.at(f, 0, 0);
       if (KIND == kStageFirst) {
-        const float u0 = A.at(f, 0, 0);
-        outs[f][i] = fmaf(cc, kv[f], u0);
-        accs[f][i] = fmaf(w, kv[f], u0);
-      } else if (KIND == kStageMid) {
-        outs[f][i] = fmaf(cc, kv[f], p.u[f]);
-        accs[f][i] = fmaf(w, kv[f], p.a[f]);
+        outs[f][i] = fmaf(cc, kv[f], y);
+      } else if (KIND == kStageLast) {
+        outs[f][i] = rk_last(kv[f], y, p.u[f], cc);
       } else {
-        outs[f][i] = fmaf(cc, kv[f], p.a[f]);
+        outs[f][i] = fmaf(cc, kv[f], p.u[f]);
+        if (KIND == kStageSecond) accs[f][i] = rk_acc(kv[f], y, p.u[f], w);
       }
     }
     if (sd) {
@@ -881,15 +881,14 @@ __device__ __forceinline__ void solid_tile(const Coef& C, const Fields& in, cons
     float* const accs[5] = {acc.svx, acc.svz, acc.ssx, acc.ssz, acc.ssxz};
 #pragma unroll
     for (int f = 0; f < 5; ++f) {
+      const float y = A.at(f, 0, 0);
       if (KIND == kStageFirst) {
-        const float u0 = A.at(f, 0, 0);
-        outs[f][i] = fmaf(cc, kv[f], u0);
-        accs[f][i] = fmaf(w, kv[f], u0);
-      } else if (KIND == kStageMid) {
-        outs[f][i] = fmaf(cc, kv[f], p.u[f]);
-        accs[f][i] = fmaf(w, kv[f], p.a[f]);
+        outs[f][i] = fmaf(cc, kv[f], y);
+      } else if (KIND == kStageLast) {
+        outs[f][i] = rk_last(kv[f], y, p.u[f], cc);
       } else {
-        outs[f][i] = fmaf(cc, kv[f], p.a[f]);
+        outs[f][i] = fmaf(cc, kv[f], p.u[f]);
+        if (KIND == kStageSecond) accs[f][i] = rk_acc(kv[f], y, p.u[f], w);
       }
     }
     if (sd) {
@@ -958,7 +957,7 @@ static cudaError_t launch_tile_one(const Coef& C, const Fields& in, const Fields
   int ntx, nbf, nbs, nbi;
   const int nshots = C.nshots > 0 ? C.nshots : 1, tr = tile_rows_of(C);
   tile_grid_of(C.nx, C.nzf, C.nzs, tr, &ntx, &nbf, &nbs, &nbi);
-  const float cc = C.rk_c[s], w = (KIND == kStageLast) ? 0.f : C.rk_w[s];
+  const float cc = C.rk_c[s], w = (KIND == kStageSecond) ? C.rk_w[s] : 0.f;
   const unsigned grid = unsigned(nbi + nbf + nbs) * unsigned(nshots);
   stage_kernel_tile<DIR, KIND, CPML><<<grid, kTileThreads, 0, st>>>(C, in, out, un, acc, s, cc, w,
                                                                     ntx, nbi, nbf, tr, nshots);
@@ -969,14 +968,16 @@ template <bool CPML>
 static cudaError_t launch_tile_bc(const Coef& C, const Fields& in, const Fields& out,
                                   const Fields& un, const Fields& acc, int stage, int dir,
                                   cudaStream_t st) {
-  const int kind = stage == 0 ? kStageFirst : (stage == 3 ? kStageLast : kStageMid);
+  const int kind = stage;  // kStageFirst .. kStageLast
   if (dir == kDirF) {
     if (kind == kStageFirst) return launch_tile_one<kDirF, kStageFirst, CPML>(C, in, out, un, acc, stage, st);
-    if (kind == kStageMid) return launch_tile_one<kDirF, kStageMid, CPML>(C, in, out, un, acc, stage, st);
+    if (kind == kStageSecond) return launch_tile_one<kDirF, kStageSecond, CPML>(C, in, out, un, acc, stage, st);
+    if (kind == kStageThird) return launch_tile_one<kDirF, kStageThird, CPML>(C, in, out, un, acc, stage, st);
     return launch_tile_one<kDirF, kStageLast, CPML>(C, in, out, un, acc, stage, st);
   }
   if (kind == kStageFirst) return launch_tile_one<kDirB, kStageFirst, CPML>(C, in, out, un, acc, stage, st);
-  if (kind == kStageMid) return launch_tile_one<kDirB, kStageMid, CPML>(C, in, out, un, acc, stage, st);
+  if (kind == kStageSecond) return launch_tile_one<kDirB, kStageSecond, CPML>(C, in, out, un, acc, stage, st);
+  if (kind == kStageThird) return launch_tile_one<kDirB, kStageThird, CPML>(C, in, out, un, acc, stage, st);
   return launch_tile_one<kDirB, kStageLast, CPML>(C, in, out, un, acc, stage, st);
 }
 

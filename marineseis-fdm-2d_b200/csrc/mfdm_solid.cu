@@ -212,18 +212,17 @@ __device__ __forceinline__ Out rhs(const SCoef& C, const SFields& S, const Acc& 
 template <int KIND>
 __device__ __forceinline__ void upd(float k, const float* in, const float* un, float* out,
                                     float* acc, size_t i, float c, float w) {
-  rk_update<KIND>(k, KIND == kStageFirst ? __ldg(in + i) : 0.f, un, out, acc, i, c, w);
+  rk_update<KIND>(k, KIND == kStageThird ? 0.f : __ldg(in + i), un, out, acc, i, c, w);
 }
 
-// The point-wise operands of one cell: U^n (`u`, the stage input itself at
-// stage 0, taken from the tile), the accumulator (`a`) and the coefficients
-// (`k`). They are loaded into registers before any store of the row -- the
+// The point-wise operands of one cell: U^n or, in the last stage, the
+// accumulator (`u`) and the coefficients (`k`). They are loaded into registers before any store of the row -- the
 // first row's before the tile barrier, so that their DRAM round trips overlap
 // the tile load (the output and accumulator pointers may alias the inputs as
 // far as the compiler knows, which would otherwise order each field's loads
 // after the previous field's stores). Loading the next row's under the
 // current row's arithmetic needs 80 registers and was slower.
-struct Pt { float u[5], a[5], k[kNCoef]; };
+struct Pt { float u[5], k[kNCoef]; };
 
 template <int KIND>
 __device__ __forceinline__ void load_pt(Pt& p, const SCoef& C, const SFields& un,
@@ -232,8 +231,8 @@ __device__ __forceinline__ void load_pt(Pt& p, const SCoef& C, const SFields& un
   const float* const pa[5] = {acc.vx, acc.vz, acc.sx, acc.sz, acc.sxz};
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    if (KIND == kStageMid) p.u[q] = __ldg(pu[q] + i);
-    if (KIND != kStageFirst) p.a[q] = pa[q][i];
+    if (KIND == kStageSecond || KIND == kStageThird) p.u[q] = __ldg(pu[q] + i);
+    if (KIND == kStageLast) p.u[q] = pa[q][i];
   }
   p.k[kCXIX] = __ldg(C.xix + i);
   p.k[kCXIZ] = __ldg(C.xiz + i);
@@ -246,8 +245,9 @@ __device__ __forceinline__ void load_pt(Pt& p, const SCoef& C, const SFields& un
   p.k[kC55] = __ldg(C.C55 + i);
 }
 
-template <int KIND>
-__device__ __forceinline__ void store5(const Out& o, const Pt& r, const SFields& out,
+// y(q): the stage input's field q at the cell.
+template <int KIND, class Y>
+__device__ __forceinline__ void store5(const Out& o, const Pt& r, const Y& y, const SFields& out,
                                        const SFields& acc, size_t i, float c, float w) {
   float* const po[5] = {out.vx, out.vz, out.sx, out.sz, out.sxz};
   float* const pa[5] = {acc.vx, acc.vz, acc.sx, acc.sz, acc.sxz};
@@ -255,13 +255,12 @@ __device__ __forceinline__ void store5(const Out& o, const Pt& r, const SFields&
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
     if (KIND == kStageFirst) {
-      po[q][i] = fmaf(c, k[q], r.u[q]);
-      pa[q][i] = fmaf(w, k[q], r.u[q]);
-    } else if (KIND == kStageMid) {
-      po[q][i] = fmaf(c, k[q], r.u[q]);
-      pa[q][i] = fmaf(w, k[q], r.a[q]);
+      po[q][i] = fmaf(c, k[q], y(q));
+    } else if (KIND == kStageLast) {
+      po[q][i] = rk_last(k[q], y(q), r.u[q], c);
     } else {
-      po[q][i] = fmaf(c, k[q], r.a[q]);
+      po[q][i] = fmaf(c, k[q], r.u[q]);
+      if (KIND == kStageSecond) pa[q][i] = rk_acc(k[q], y(q), r.u[q], w);
     }
   }
 }
@@ -282,10 +281,6 @@ __device__ __forceinline__ void rows(const SCoef& C, const SFields& in, const SF
     auto A = [&](int q, int dz, int dx) { return tile[q][lz + dz][3 + threadIdx.x + dx]; };
     const size_t i = (size_t)iz * P + ix;
     if (k > 0) load_pt<KIND>(p, C, un, acc, i);
-    if (KIND == kStageFirst) {
-#pragma unroll
-      for (int q = 0; q < 5; ++q) p.u[q] = A(q, 0, 0);
-    }
     auto K = [&](int cf) { return p.k[cf]; };
     Out o = rhs<DIR, IN, CPML>(C, in, A, K, iz, ix);
     if (!IN) {
@@ -297,7 +292,7 @@ __device__ __forceinline__ void rows(const SCoef& C, const SFields& in, const SF
         o.sz += q;
       }
     }
-    store5<KIND>(o, p, out, acc, i, c, w);
+    store5<KIND>(o, p, [&](int q) { return A(q, 0, 0); }, out, acc, i, c, w);
     if (!IN && min(ix - 3, nx - 4 - ix) < npd) {
       const size_t si = (size_t)iz * C.Ps + xstrip_col(ix, nx, npd);
       upd<KIND>(o.XV0, in.x[0], un.x[0], out.x[0], acc.x[0], si, c, w);
@@ -392,7 +387,7 @@ template <int DIR, int KIND>
 cudaError_t launch_t(const SCoef& C, const SFields& in, const SFields& out, const SFields& un,
                      const SFields& acc, int s, cudaStream_t st) {
   const dim3 grid(unsigned((C.nx - 6 + kBX - 1) / kBX), unsigned((C.nz - 6 + kTZ - 1) / kTZ));
-  const float c = C.rk_c[s], w = KIND == kStageLast ? 0.f : C.rk_w[s];
+  const float c = C.rk_c[s], w = KIND == kStageSecond ? C.rk_w[s] : 0.f;
   if (C.cpml)
     k_stage<DIR, KIND, true><<<grid, dim3(kBX, kBY), 0, st>>>(C, in, out, un, acc, s, c, w);
   else
@@ -406,12 +401,14 @@ cudaError_t launch_stage(const SCoef& C, const SFields& in, const SFields& out, 
                          const SFields& acc, int stage, int dir, cudaStream_t st) {
   if (dir == kDirF) {
     if (stage == 0) return launch_t<kDirF, kStageFirst>(C, in, out, un, acc, stage, st);
-    if (stage == 3) return launch_t<kDirF, kStageLast>(C, in, out, un, acc, stage, st);
-    return launch_t<kDirF, kStageMid>(C, in, out, un, acc, stage, st);
+    if (stage == 1) return launch_t<kDirF, kStageSecond>(C, in, out, un, acc, stage, st);
+    if (stage == 2) return launch_t<kDirF, kStageThird>(C, in, out, un, acc, stage, st);
+    return launch_t<kDirF, kStageLast>(C, in, out, un, acc, stage, st);
   }
   if (stage == 0) return launch_t<kDirB, kStageFirst>(C, in, out, un, acc, stage, st);
-  if (stage == 3) return launch_t<kDirB, kStageLast>(C, in, out, un, acc, stage, st);
-  return launch_t<kDirB, kStageMid>(C, in, out, un, acc, stage, st);
+  if (stage == 1) return launch_t<kDirB, kStageSecond>(C, in, out, un, acc, stage, st);
+  if (stage == 2) return launch_t<kDirB, kStageThird>(C, in, out, un, acc, stage, st);
+  return launch_t<kDirB, kStageLast>(C, in, out, un, acc, stage, st);
 }
 
 cudaError_t launch_finish(const SCoef& C, const SFields& U, cudaStream_t st) {
