@@ -70,8 +70,8 @@ typedef struct mfdm_info {
   long long cells;                /* nx * (nz_f + nz_s): cells updated per step */
   long long device_bytes;         /* device memory held by the handle */
   int nshots;                     /* shots stepped together (1 unless opened with mfdm_open_batch) */
-  int seg_rows;                   /* rows per segment block of the stage launches */
-  int blocks_per_sm;              /* stage kernel build in use: 2 or 3 (TMA rings), 4 (tiles) */
+  int seg_rows;                   /* rows per interior tile of the stage launches */
+  int blocks_per_sm;              /* stage kernel build in use: 2, 3 or 4 (mfdm_set_blocks_per_sm) */
 } mfdm_info;
 
 /* Field ids for mfdm_get_field / mfdm_set_field. */
@@ -130,8 +130,9 @@ int mfdm_step(mfdm_model* m, int nsteps);
  * with CUDA events on the handle's stream: *total_ms for the whole run. With
  * per_kernel != 0 the steps are launched one by one (back to back, outside the
  * graph) with an event between consecutive kernels, and kernel_ms[0..3] receive
- * the summed time of the four RK stage launches and kernel_ms[4] that of the
- * filter/receiver launch. */
+ * the summed time of the four RK stage launches (the last one filters the
+ * interface rows and samples the receivers) and kernel_ms[4] what passes between
+ * the last one's event and the step's end. */
 int mfdm_time_steps(mfdm_model* m, int nsteps, int per_kernel, float* total_ms, float* kernel_ms);
 
 /* Waits for the handle's stream. */
@@ -177,30 +178,27 @@ int mfdm_batch_get_records(mfdm_model* m, int shot, int first, int count, float*
 int mfdm_batch_get_field(mfdm_model* m, int shot, int field, float* host);
 
 /* ---- tile shape ---------------------------------------------------------
- * A stage launch covers each medium with segment blocks of 64 columns by
- * `seg_rows` rows. Small grids want short segments (more blocks than SMs),
- * large ones long segments (fewer halo re-reads). The reference launches
- * fixed 16x16 blocks (src/pml_fs_kernels.cu:533-622) and has no tuner. */
+ * A stage launch covers the interior of each medium with tiles of 32 columns by
+ * `seg_rows` rows. Small grids want short tiles (more blocks), large ones tall
+ * tiles (fewer halo rows staged twice). The reference launches fixed 16x16
+ * blocks (src/pml_fs_kernels.cu:533-622) and has no tuner. */
 
-/* Sets the segment height: a multiple of 4 in [4, 128], or 0 for the default
- * (24 from 6 M cells per launch, counting every shot of a batch, 8 below; the
- * tile build, mfdm_set_blocks_per_sm 4, rounds it up to a multiple of 8 and
- * caps it at 48, 16 by default). Results do not depend on it beyond FP32
- * rounding of the last bit. */
+/* Sets the tile height: a multiple of 4 in [4, 128] (the kernels round it up
+ * to a multiple of 8 and cap it at 48), or 0 for the default (8 rows below 0.2 M
+ * cells per launch, counting every shot of a batch, 16 below 0.5 M, 24 below
+ * 4 M, 32 above). Results do not depend on it beyond FP32 rounding of the last
+ * bit. */
 int mfdm_set_tile(mfdm_model* m, int seg_rows);
 
-/* Selects the stage kernel build: 2 resident blocks per SM (deeper TMA rings,
- * 96 registers) or 3 (shallower rings, 72 registers, more bytes in flight per
- * SM: faster on large grids, slower on small ones); 4: the tile build (no
- * rings: 256-thread blocks stage 32 x 16 cells and their halo in shared
- * memory with plain loads while the point-wise operands of each thread's
- * first row are already in flight); 0 (default): the 3-block build. Results
- * agree to FP32 rounding. */
+/* Selects the stage kernel build by its register budget: 2 or 3 resident blocks
+ * per SM (128 or 80 registers: the strip and interface paths spill little, so
+ * a small grid's few blocks finish sooner), 4: five blocks per SM (48
+ * registers: more loads in flight, faster on large grids); 0 (default): 3 below
+ * 0.5 M cells per launch, 4 from there. Results agree to FP32 rounding. */
 int mfdm_set_blocks_per_sm(mfdm_model* m, int blocks);
 
-/* Times every candidate segment height with both ring builds (2 and 3 blocks
- * per SM), and the tile build, on this handle's model and shots
- * (a few steps each, CUDA events on the handle's stream), keeps the fastest and
+/* Times every candidate tile height with every build on this handle's model and
+ * shots (a few steps each, CUDA events on the handle's stream), keeps the fastest and
  * writes it to *seg_rows (may be NULL). The choice is cached per device, grid
  * shape, PML width, boundary type and shot count, so a second handle of the
  * same shape is not timed again. The timing steps change the state: on return
@@ -423,13 +421,11 @@ int mfdm_dispersion_image(const float* gather, int nt, int ntr, const double* of
  * fluid grid is rejected (src_x < 0: no source). The Ricker and PML tables come
  * from the same host functions as an open handle's, so the results are
  * bit-identical to mfdm_step on the same model. The first call on a device
- * resolves that array's address and configures the kernels there, so make it
- * before any stream capture; after cudaDeviceReset of that device, do not call
+ * resolves that array's address there, so make it before any stream capture; after cudaDeviceReset of that device, do not call
  * it again in the same process. Calls share the array and it keeps the last
  * call's contents: the ADE memory carries from one call to the next, so start
  * a run with it == 0 (which clears it) and continue one model with consecutive
- * time indices; calls that overlap on the GPU race. A pipeline wait that times
- * out returns MFDM_ERR_CUDA and leaves the state arrays undefined. No receiver
+ * time indices; calls that overlap on the GPU race. No receiver
  * buffer: read the state arrays. */
 int mfdm_step_noalloc(const mfdm_device_model* dm, int it, int nsteps, void* stream);
 

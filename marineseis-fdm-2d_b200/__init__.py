@@ -371,16 +371,15 @@ class Solver:
 
     # -- tile shape -----------------------------------------------------------
     def set_tile(self, seg_rows: int):
-        """Rows per segment block of the stage launches (multiple of 4 in [4, 128]; 0: 24)."""
+        """Rows per interior tile of the stage launches (multiple of 4 in [4, 128]; 0: by size)."""
         _check(self._lib.mfdm_set_tile(self._h, int(seg_rows)))
 
     def set_blocks_per_sm(self, blocks: int):
-        """Stage kernel build: 2 or 3 resident blocks per SM (TMA rings), 4 (tiles), 0 the
-        default 3 (mfdm_set_blocks_per_sm)."""
+        """Stage kernel build: 2, 3 (latency) or 4 (throughput), 0: by size (mfdm_set_blocks_per_sm)."""
         _check(self._lib.mfdm_set_blocks_per_sm(self._h, int(blocks)))
 
     def autotune(self) -> int:
-        """Times the candidate segment heights, keeps the fastest and returns it.
+        """Times the candidate tile heights and builds, keeps the fastest and returns it.
         Leaves every shot at rest at step 0 (mfdm_autotune)."""
         seg = ctypes.c_int()
         _check(self._lib.mfdm_autotune(self._h, ctypes.byref(seg)))

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import glob
 import os
+from concurrent.futures import ThreadPoolExecutor
 import shutil
 import subprocess
 
@@ -17,6 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libmfdm.so")
 CLI = os.path.join(HERE, "bin", "main_debug")
+OBJ = os.path.join(HERE, "build")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC"] + ARCH
 
@@ -46,10 +48,17 @@ def build(verbose: bool = False, force: bool = False) -> str:
     deps.append(os.path.join(ROOT, "include", "mfdm.h"))
     lib_srcs = [s for s in _sources() if not s.endswith("main_debug.cpp")]
     if force or _stale(LIB, deps):
-        cmd = [nvcc] + NVCC_FLAGS + ["-shared", "-o", LIB] + lib_srcs
-        if verbose:
-            print(" ".join(cmd))
-        subprocess.run(cmd, check=True)
+        os.makedirs(OBJ, exist_ok=True)
+        objs = [os.path.join(OBJ, os.path.splitext(os.path.basename(s))[0] + ".o") for s in lib_srcs]
+
+        def run(cmd):
+            if verbose:
+                print(" ".join(cmd))
+            subprocess.run(cmd, check=True)
+
+        with ThreadPoolExecutor(max(1, min(len(lib_srcs), os.cpu_count() or 1))) as pool:
+            list(pool.map(run, [[nvcc] + NVCC_FLAGS + ["-c", s, "-o", o] for s, o in zip(lib_srcs, objs)]))
+        run([nvcc] + ARCH + ["-shared", "-o", LIB] + objs)
     os.makedirs(os.path.dirname(CLI), exist_ok=True)
     if force or _stale(CLI, [LIB, os.path.join(CSRC, "main_debug.cpp")]):
         cmd = [nvcc] + ARCH + ["-O2", "-std=c++17", os.path.join(CSRC, "main_debug.cpp"), "-L" + HERE,

@@ -591,6 +591,7 @@ __global__ void __launch_bounds__(128, 6) k_grad_cells(Coef C, SetLayout L, Fiel
   }
   const bool side = min(ix - 3, nx - 4 - ix) < npd;
   const int scol = side ? xstrip_col(ix, nx, npd) : 0;
+  const float4 px = side ? __ldg(C.pmlx + ix) : make_float4(0.f, 0.f, 0.f, 0.f);
   const int nfr = nzf - 4;
   const int row = blockIdx.y - 1;
   if (row < nfr) {
@@ -605,10 +606,11 @@ __global__ void __launch_bounds__(128, 6) k_grad_cells(Coef C, SetLayout L, Fiel
     const bool top = CPML && iz <= npd + 2;
     if (top)
       for (int q = 0; q < 4; ++q) zade[q] = __ldg(Y.fz[q] + (size_t)(iz - 3) * P + ix);
+    const float4 pzf = top ? __ldg(C.pmlzf + iz) : make_float4(0.f, 0.f, 0.f, 0.f);
     const FluidCoefs cf{__ldg(C.xix + g), __ldg(C.xiz + g), __ldg(C.zex + g), __ldg(C.zez + g),
                         1.0f, 1.0f};
     FluidGlobal A{Y.fvx, Y.fvz, Y.fp, g, P};
-    const FluidK o = fluid_rhs<DIR, false, CPML>(C, A, iz, ix, side, ade, cf, top, zade);
+    const FluidK o = fluid_rhs<DIR, false, CPML>(C, A, iz, ix, side, ade, cf, px, top, zade, pzf);
     // velocity terms carry 1/rho, the pressure term K
     G.rf[g] = grf + (double(__ldg(KB.fvx + g)) * o.vx + double(__ldg(KB.fvz + g)) * o.vz);
     G.K[g] = gK + double(__ldg(KB.fp + g)) * o.p;
@@ -620,6 +622,7 @@ __global__ void __launch_bounds__(128, 6) k_grad_cells(Coef C, SetLayout L, Fiel
   const size_t m = (size_t)iz * P + ix, g = m + (size_t)(nzf - 1) * P;
   const int zb0 = nzs - 3 - npd;
   const bool bottom = iz >= zb0;
+  const float4 pz = bottom ? __ldg(C.pmlz + iz) : make_float4(0.f, 0.f, 0.f, 0.f);
   const double gc11 = G.c11[m], gc33 = G.c33[m], gc55 = G.c55[m], grs = G.rs[m], gc13 = G.c13[m];
   float xade[4] = {0.f, 0.f, 0.f, 0.f}, zade[4] = {0.f, 0.f, 0.f, 0.f};
   if (side)
@@ -633,7 +636,7 @@ __global__ void __launch_bounds__(128, 6) k_grad_cells(Coef C, SetLayout L, Fiel
                ksz = __ldg(KB.ssz + m), ksxz = __ldg(KB.ssxz + m);
   // C11, C33, C55 and 1/rho each reach a different output; C13 reaches sx and sz
   const SolidK o1 = solid_rhs<DIR, false, CPML>(C, A, iz, ix, side, bottom, xade, zade,
-                                                SolidCoefs{xix, xiz, zex, zez, 1.f, 1.f, 0.f, 1.f, 1.f});
+                                                SolidCoefs{xix, xiz, zex, zez, 1.f, 1.f, 0.f, 1.f, 1.f}, px, pz);
   double t13;
   if (!side && !bottom) {
     // off the PML strips the stress RHS is sx = C11 X + C13 Z, sz = C13 X + C33 Z,
@@ -641,7 +644,7 @@ __global__ void __launch_bounds__(128, 6) k_grad_cells(Coef C, SetLayout L, Fiel
     t13 = ksx * o1.sz + ksz * o1.sx;
   } else {
     const SolidK o2 = solid_rhs<DIR, false, CPML>(C, A, iz, ix, side, bottom, xade, zade,
-                                                  SolidCoefs{xix, xiz, zex, zez, 0.f, 0.f, 1.f, 0.f, 0.f});
+                                                  SolidCoefs{xix, xiz, zex, zez, 0.f, 0.f, 1.f, 0.f, 0.f}, px, pz);
     t13 = ksx * o2.sx + ksz * o2.sz;
   }
   G.c11[m] = gc11 + ksx * o1.sx;
@@ -680,12 +683,16 @@ __device__ __forceinline__ void grad_iface(const Coef& C, const Fields& Y, const
               fzez = __ldg(C.zez + fi);
   const float sxix = __ldg(C.xix + gs), sxiz = __ldg(C.xiz + gs), szex = __ldg(C.zex + gs),
               szez = __ldg(C.zez + gs);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 px = side ? __ldg(C.pmlx + ix) : zero, pz = bottom ? __ldg(C.pmlz) : zero,
+               pzf = ftop ? __ldg(C.pmlzf + nzf - 1) : zero;
   const FluidK of = fluid_rhs<DIR, false, CPML>(C, Af, nzf - 1, ix, side, fade,
-                                                FluidCoefs{fxix, fxiz, fzex, fzez, 1.f, 1.f}, ftop, ztop);
+                                                FluidCoefs{fxix, fxiz, fzex, fzez, 1.f, 1.f}, px, ftop, ztop,
+                                                pzf);
   const SolidK o1 = solid_rhs<DIR, false, CPML>(C, As, 0, ix, side, bottom, xade, zade,
-                                                SolidCoefs{sxix, sxiz, szex, szez, 1.f, 1.f, 0.f, 1.f, 1.f});
+                                                SolidCoefs{sxix, sxiz, szex, szez, 1.f, 1.f, 0.f, 1.f, 1.f}, px, pz);
   const SolidK o2 = solid_rhs<DIR, false, CPML>(C, As, 0, ix, side, bottom, xade, zade,
-                                                SolidCoefs{sxix, sxiz, szex, szez, 0.f, 0.f, 1.f, 0.f, 0.f});
+                                                SolidCoefs{sxix, sxiz, szex, szez, 0.f, 0.f, 1.f, 0.f, 0.f}, px, pz);
   const float kb[8] = {__ldg(KB.fvx + fi), __ldg(KB.fvz + fi), __ldg(KB.fp + fi), __ldg(KB.svx + si),
                        __ldg(KB.svz + si), __ldg(KB.ssx + si), __ldg(KB.ssz + si), __ldg(KB.ssxz + si)};
   const float2 n = __ldg(C.nrm + ix);

@@ -1,120 +1,25 @@
-// Bulk asynchronous copies (the TMA engine's non-tensor form) and mbarrier
-// waits for sm_100a, as hand-written inline PTX.
-//
-// Every wait is bounded: after kWaitNs nanoseconds of %globaltimer it gives
-// up and reports failure, so a mis-counted transaction can never hang a GPU;
-// the kernel then records the failure in its status word and returns.
+// Asynchronous global -> shared copies, as hand-written inline PTX.
 #pragma once
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace mfdm {
 
-constexpr unsigned long long kWaitNs = 1000000000ull;  // 1 s
-
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
+// Global -> shared asynchronous copy of 16 bytes (zeros when !ok: nothing is
+// read), committed and awaited per thread.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0)
                : "memory");
 }
-
-// Makes initialised barriers visible to the async (copy) proxy.
-__device__ __forceinline__ void mbar_fence_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+__device__ __forceinline__ void cp_async_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
 }
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
-// Suspend-time hint of mbarrier.try_wait in ns; 0 (the default) leaves the
-// suspension to the hardware's own time limit. Measured on the stage kernels:
-// no hint runs 0.7-1.9 % faster than a 20 us hint (1 us and 1 ms: as 20 us).
-#ifndef MFDM_WAIT_HINT_NS
-#define MFDM_WAIT_HINT_NS 0
-#endif
-
-// try_wait suspends the thread in hardware until the phase completes or a
-// time limit (the hint, or the hardware's) elapses, instead of spinning on
-// issue slots.
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-  uint32_t ok;
-#if MFDM_WAIT_HINT_NS > 0
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity), "r"(unsigned(MFDM_WAIT_HINT_NS))
-      : "memory");
-#else
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-#endif
-  return ok != 0;
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Waits for the phase with the given parity to complete; false after kWaitNs.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
-  for (;;) {
-    for (int i = 0; i < 8; ++i)
-      if (mbar_try_wait(bar, parity)) return true;
-    if (global_ns() - t0 > kWaitNs) return false;
-  }
-}
-
-// Global -> shared bulk copy completing on `bar` (addresses 16-byte aligned,
-// bytes a multiple of 16).
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_addr(dst)),
-      "l"(src), "r"(bytes), "r"(smem_addr(bar))
-      : "memory");
-}
-
-// 3-D tiled tensor load (TMA) of one box into shared memory, completing on
-// `bar`; out-of-range elements (negative or past-the-end coordinates) read 0.
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_addr(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_addr(bar))
-      : "memory");
-}
-
-// 4-D tiled tensor load (the fourth coordinate selects the shot).
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int x, int y, int z,
-                                            int w, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_addr(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_addr(bar))
-      : "memory");
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 }  // namespace mfdm

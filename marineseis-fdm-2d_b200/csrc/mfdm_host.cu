@@ -56,13 +56,6 @@ int fail(int code, const std::string& msg) {
 
 constexpr int kGraphSteps = 32;  // steps per captured graph (must be even)
 
-// 5x5 source weights (src/elements.cu:34-40) and the interface filter (src/elements.cu:30-33).
-const float kSrcW[25] = {0.0030f, 0.0133f, 0.0219f, 0.0133f, 0.0030f, 0.0133f, 0.0596f,
-                         0.0983f, 0.0596f, 0.0133f, 0.0219f, 0.0983f, 0.1621f, 0.0983f,
-                         0.0219f, 0.0133f, 0.0596f, 0.0983f, 0.0596f, 0.0133f, 0.0030f,
-                         0.0133f, 0.0219f, 0.0133f, 0.0030f};
-const float kW7[7] = {1.1e-13f, 1.678e-06f, 0.03419f, 0.93163f, 0.03419f, 1.678e-06f, 1.1e-13f};
-
 struct HostModel {
   int nx = 0, nzf = 0, nzs = 0;
   float fpeak = 0.f, dt = 0.f;
@@ -151,6 +144,7 @@ struct mfdm_model {
   int P = 0, Ps = 0, nz = 0, gap = 1;
   int isrc = 0;
   int host_step = 0;
+  int dev_step = 0;  // the device step counter's value once the stream gets there
   char* dmem = nullptr;
   size_t dbytes = 0;
   Fields S[4];  // U, stage A, stage B, accumulator
@@ -161,9 +155,6 @@ struct mfdm_model {
   int rec_cap = 0;
   cudaGraphExec_t graph = nullptr;
   unsigned gen = 0;  // bumped whenever captured launches go stale (groups recapture)
-  // TMA descriptors: per RK set (U, A, B, acc) the stencil box and the
-  // point-wise box of the fluid and solid blocks, and the coefficient blocks.
-  CUtensorMap fst[4], sst[4], fpw[4], spw[4], fco, sco;
   float* fcoef = nullptr;  // [6][nz_f][P]: xi_x, xi_z, ze_x, ze_z, rho, K
   float* scoef = nullptr;  // [9][nz_s][P]: xi_x, xi_z, ze_x, ze_z, rho, C11, C13, C33, C55
   AdjointState* adj = nullptr;  // adjoint operators and buffers (mfdm_adjoint_*)
@@ -189,15 +180,6 @@ struct AdjointState {
   size_t seg_steps = 0;    // while this one is reversed (when the memory allows)
   float* keep = nullptr;   // stage inputs of the last `nkeep` segments, kept by the forward pass
   size_t keep_floats = 0;
-  // TMA maps of every step slot's four stage-input sets (stencil boxes) and of
-  // its first set as U^n (point-wise boxes), per buffer of slots (keep, seg,
-  // seg2): kept and recomputed steps run their stages in place in the slots
-  struct SlotMaps { CUtensorMap fst[4], sst[4], fun, sun; };
-  struct SlotTable {
-    const float* base = nullptr;
-    std::vector<SlotMaps> maps;
-  };
-  SlotTable keep_tab, seg_tab[2];
   int nkeep = 0;
   float* res = nullptr;    // residual samples [ns][3][nx]
   float* inner = nullptr;  // second-level checkpoints of one segment
@@ -360,45 +342,6 @@ void fill_src_table(const HostModel& h, float fpeak, int steps, float* amp) {
   }
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link).
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// Map of a block [nf][rows][P] of floats read in boxes of box_x columns, kStageR
-// rows and all nf fields. Point-wise maps land as [field][row][col] (dimensions
-// column, row, field); stencil maps (rows_outer) land as [row][field][col]
-// (dimensions column, field, row), so consecutive chunks stack into one
-// row-contiguous ring.
-// With nshots > 0 the map has a fourth dimension, the shot, of stride shot_bytes.
-int encode_block(CUtensorMap* map, const float* base, int P, int rows, int nf, int box_x,
-                 bool rows_outer, int nshots = 0, size_t shot_bytes = 0) {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    MFDM_CU(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q));
-    if (!p || q != cudaDriverEntryPointSuccess)
-      return fail(MFDM_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-    fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  const cuuint64_t row_stride = cuuint64_t(P) * 4, field_stride = cuuint64_t(rows) * P * 4;
-  const cuuint64_t dims[4] = {cuuint64_t(P), cuuint64_t(rows_outer ? nf : rows),
-                              cuuint64_t(rows_outer ? rows : nf), cuuint64_t(nshots > 0 ? nshots : 1)};
-  const cuuint64_t strides[3] = {rows_outer ? field_stride : row_stride,
-                                 rows_outer ? row_stride : field_stride, cuuint64_t(shot_bytes)};
-  const cuuint32_t box[4] = {cuuint32_t(box_x), cuuint32_t(rows_outer ? nf : mfdm::kStageR),
-                             cuuint32_t(rows_outer ? mfdm::kStageR : nf), 1};
-  const cuuint32_t es[4] = {1, 1, 1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, nshots > 0 ? 4 : 3,
-                        const_cast<float*>(base), dims,
-                        strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(MFDM_ERR_CUDA, "tensor map encoding failed (" + std::to_string(int(r)) + ")");
-  return MFDM_OK;
-}
-
 void release_graph(mfdm_model* m) {
   ++m->gen;
   if (m->graph) {
@@ -449,32 +392,25 @@ int ensure_capacity(mfdm_model* m, int steps) {
   return MFDM_OK;
 }
 
-// Enqueues the five launches of one step. With `ev` (6 events) an event is
-// recorded before the first launch and after every launch.
-int enqueue_step(mfdm_model* m, int it, cudaStream_t st, cudaEvent_t* ev = nullptr) {
+// Enqueues the launches of one step of time index `it`. With `ev` (6 events) an
+// event is recorded before the first launch, after every stage launch and at
+// the step's end. `captured`: the time index is the device step counter + it.
+int enqueue_step(mfdm_model* m, int it, cudaStream_t st, cudaEvent_t* ev = nullptr,
+                 bool captured = false) {
   const int d0 = (it & 1) ? mfdm::kDirB : mfdm::kDirF, d1 = 1 - d0;
   const Fields &U = m->S[0], &A = m->S[1], &B = m->S[2], &Acc = m->S[3];
-  const Coef& C = m->C;
+  Coef C = m->C;
+  if (!captured) C.step = nullptr;
+  C.it_off = it;
   // stage s reads in[s] and writes out[s]: U -> A -> B -> A -> U
   const Fields* in[4] = {&U, &A, &B, &A};
   const Fields* out[4] = {&A, &B, &A, &U};
-  const int in_set[4] = {0, 1, 2, 1};
   const int dir[4] = {d0, d1, d0, d1};
   if (ev) MFDM_CU(cudaEventRecord(ev[0], st));
   for (int s = 0; s < 4; ++s) {
-    mfdm::StageMaps maps;
-    maps.fin = m->fst[in_set[s]];
-    maps.sin = m->sst[in_set[s]];
-    maps.fun = m->fpw[0];
-    maps.sun = m->spw[0];
-    maps.facc = m->fpw[3];
-    maps.sacc = m->spw[3];
-    maps.fcoef = m->fco;
-    maps.scoef = m->sco;
-    MFDM_CU(mfdm::launch_stage(C, *in[s], *out[s], U, Acc, maps, s, dir[s], st));
+    MFDM_CU(mfdm::launch_stage(C, *in[s], *out[s], U, Acc, s, dir[s], st));
     if (ev) MFDM_CU(cudaEventRecord(ev[s + 1], st));
   }
-  MFDM_CU(mfdm::launch_finish(C, U, st));
   if (ev) MFDM_CU(cudaEventRecord(ev[5], st));
   return MFDM_OK;
 }
@@ -486,7 +422,9 @@ int capture_graph(mfdm_model* m) {
   cudaGraph_t g = nullptr;
   MFDM_CU(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
   int rc = MFDM_OK;
-  for (int k = 0; k < kGraphSteps && rc == MFDM_OK; ++k) rc = enqueue_step(m, k, m->stream);
+  for (int k = 0; k < kGraphSteps && rc == MFDM_OK; ++k) rc = enqueue_step(m, k, m->stream, nullptr, true);
+  if (rc == MFDM_OK && mfdm::launch_advance_step(m->C, kGraphSteps, m->stream) != cudaSuccess)
+    rc = fail(MFDM_ERR_CUDA, "graph capture: step counter");
   cudaError_t e = cudaStreamEndCapture(m->stream, &g);
   if (rc != MFDM_OK) {
     if (g) cudaGraphDestroy(g);
@@ -499,15 +437,9 @@ int capture_graph(mfdm_model* m) {
   return MFDM_OK;
 }
 
-// Maps a kernel status word to an error: bit 2 (value 2) is a pipeline wait
-// that timed out, after which the handle's state is undefined (reopen it);
-// bit 1 a non-finite value.
+// Maps a kernel status word to an error.
 int status_error(int st, const char* nonfinite_msg) {
-  if (st & 2)
-    return fail(MFDM_ERR_CUDA,
-                "a stage kernel pipeline wait timed out; the handle's state is undefined, reopen it");
-  if (st) return fail(MFDM_ERR_NONFINITE, nonfinite_msg);
-  return MFDM_OK;
+  return st ? fail(MFDM_ERR_NONFINITE, nonfinite_msg) : MFDM_OK;
 }
 
 int check_status(mfdm_model* m) {
@@ -634,13 +566,11 @@ int build(mfdm_model* m, HostModel&& h, int device, const std::vector<ShotCfg>* 
   MFDM_CU(cudaGetDeviceCount(&ndev));
   if (device < 0 || device >= ndev) return fail(MFDM_ERR_ARG, "no such CUDA device");
   MFDM_CU(cudaSetDevice(device));
-  MFDM_CU(mfdm::configure_device());
-  MFDM_CU(mfdm::upload_constants(kSrcW, kW7));
   MFDM_CU(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
 
   const int nx = h.nx, nzf = h.nzf, nzs = h.nzs, nz = nzf + nzs - 1;
-  // pitch: 128-byte rows, and never narrower than the 72-column TMA stencil box
-  const int P = round_up(std::max(nx, mfdm::kStageSW), 32), Ps = round_up(std::max(2 * h.npd, 1), 4);
+  // pitch: 128-byte rows
+  const int P = round_up(std::max(nx, mfdm::kMinPitch), 32), Ps = round_up(std::max(2 * h.npd, 1), 4);
   const int npdr = std::max(h.npd, 1);
   m->P = P; m->Ps = Ps; m->nz = nz;
 
@@ -660,8 +590,7 @@ int build(mfdm_model* m, HostModel&& h, int device, const std::vector<ShotCfg>* 
   const size_t shared = off;
   // One region per shot (equal sizes, so shot b's buffers are b regions after
   // shot 0's): each RK set's fluid block [3][nz_f][P] and solid block
-  // [5][nz_s][P] (the TMA boxes span the fields), the ADE strips, the PML
-  // factors and the interface rows.
+  // [5][nz_s][P], the ADE strips and the PML factors.
   size_t roff = 0;
   auto rtake = [&](size_t nfloats) {
     const size_t o = roff;
@@ -678,7 +607,7 @@ int build(mfdm_model* m, HostModel&& h, int device, const std::vector<ShotCfg>* 
     for (int q = 0; q < 4; ++q) o_fza[s][q] = rtake(h.bdy == 1 ? size_t(npdr) * P : 1);
   }
   const size_t o_pmlx = rtake(size_t(nx) * 4), o_pmlz = rtake(size_t(nzs) * 4),
-               o_pmlzf = rtake(size_t(nzf) * 4), o_ipre = rtake(size_t(8) * P);
+               o_pmlzf = rtake(size_t(nzf) * 4);
   m->region = roff;
   off = shared + roff * size_t(m->nshots);
   m->dbytes = off;
@@ -713,10 +642,9 @@ int build(mfdm_model* m, HostModel&& h, int device, const std::vector<ShotCfg>* 
   C.pmlzf = reinterpret_cast<const float4*>(R(o_pmlzf));
   C.cpml = h.bdy == 1 ? 1 : 0;
   C.nrm = reinterpret_cast<const float2*>(F(o_nrm));
-  C.ipre = R(o_ipre);
   int* misc = reinterpret_cast<int*>(F(o_misc));
   C.step = misc;
-  C.done = reinterpret_cast<unsigned*>(misc + 1);
+  C.it_off = 0;
   C.status = misc + 2;
   C.nshots = m->nshots;
   C.shot_stride = roff / sizeof(float);
@@ -734,16 +662,6 @@ int build(mfdm_model* m, HostModel&& h, int device, const std::vector<ShotCfg>* 
                             cudaMemcpyHostToDevice, m->stream));
     C.src_pos = reinterpret_cast<const int2*>(m->d_srcpos);
   }
-  for (int s = 0; s < 4; ++s) {
-    if ((rc = encode_block(&m->fst[s], R(o_fb[s]), P, nzf, 3, mfdm::kStageSW, true, m->nshots, roff)) ||
-        (rc = encode_block(&m->sst[s], R(o_sb[s]), P, nzs, 5, mfdm::kStageSW, true, m->nshots, roff)) ||
-        (rc = encode_block(&m->fpw[s], R(o_fb[s]), P, nzf, 3, mfdm::kStageTX, false, m->nshots, roff)) ||
-        (rc = encode_block(&m->spw[s], R(o_sb[s]), P, nzs, 5, mfdm::kStageTX, false, m->nshots, roff)))
-      return rc;
-  }
-  if ((rc = encode_block(&m->fco, m->fcoef, P, nzf, 6, mfdm::kStageTX, false)) ||
-      (rc = encode_block(&m->sco, m->scoef, P, nzs, 9, mfdm::kStageTX, false)))
-    return rc;
   if ((rc = upload_model(m, h)) != MFDM_OK) return rc;
   MFDM_CU(mfdm::launch_set_step(m->C, 0, m->stream));
   MFDM_CU(cudaStreamSynchronize(m->stream));
@@ -784,8 +702,7 @@ int open_common(HostModel&& h, int device, mfdm_model** out,
 
 int field_ptr(mfdm_model* m, int field, float** p, int* rows, int shot = 0);
 
-// Zeroes every shot's RK sets (state, stage buffers, accumulator), ADE strips
-// and interface rows; the coefficients and the PML tables stay.
+// Zeroes every shot's RK sets (state, stage buffers, accumulator) and ADE strips; the coefficients and the PML tables stay.
 int clear_state(mfdm_model* m) {
   const size_t pitch = m->region, h = size_t(m->nshots);
   const size_t nf = size_t(m->cfg.nzf) * m->P, ns = size_t(m->cfg.nzs) * m->P;
@@ -806,7 +723,6 @@ int clear_state(mfdm_model* m) {
                                   m->stream));
     }
   }
-  MFDM_CU(cudaMemset2DAsync(m->C.ipre, pitch, 0, size_t(8) * m->P * sizeof(float), h, m->stream));
   return MFDM_OK;
 }
 
@@ -817,6 +733,7 @@ int rewind(mfdm_model* m) {
   MFDM_CU(cudaMemsetAsync(m->C.status, 0, sizeof(int), m->stream));
   m->host_step = 0;
   MFDM_CU(mfdm::launch_set_step(m->C, 0, m->stream));
+  m->dev_step = 0;
   MFDM_CU(cudaStreamSynchronize(m->stream));
   return MFDM_OK;
 }
@@ -871,10 +788,6 @@ int field_ptr(mfdm_model* m, int field, float** p, int* rows, int shot) {
 namespace mfdm {
 // Shared with other translation units of the library.
 int set_error(int code, const char* msg) { return fail(code, msg); }
-int encode_block_map(CUtensorMap* map, const float* base, int P, int rows, int nf, int box_x,
-                     bool rows_outer, int nshots, size_t shot_bytes) {
-  return encode_block(map, base, P, rows, nf, box_x, rows_outer, nshots, shot_bytes);
-}
 }  // namespace mfdm
 
 extern "C" {
@@ -911,13 +824,24 @@ int desc_to_host(const mfdm_desc* d, HostModel& h) {
   return MFDM_OK;
 }
 
+// Brings the device step counter, which only captured steps read and advance,
+// to the next time index.
+int sync_step(mfdm_model* m, cudaStream_t st) {
+  if (m->dev_step == m->host_step) return MFDM_OK;
+  MFDM_CU(mfdm::launch_set_step(m->C, m->host_step, st));
+  m->dev_step = m->host_step;
+  return MFDM_OK;
+}
+
 int enqueue_steps(mfdm_model* m, int nsteps) {
   int rc;
   while (nsteps > 0) {
     if ((m->host_step & 1) == 0 && nsteps >= kGraphSteps) {
       if (!m->graph && (rc = capture_graph(m)) != MFDM_OK) return rc;
+      if ((rc = sync_step(m, m->stream)) != MFDM_OK) return rc;
       MFDM_CU(cudaGraphLaunch(m->graph, m->stream));
       m->host_step += kGraphSteps;
+      m->dev_step = m->host_step;
       nsteps -= kGraphSteps;
     } else {
       if ((rc = enqueue_step(m, m->host_step, m->stream)) != MFDM_OK) return rc;
@@ -1000,7 +924,6 @@ int mfdm_update_rk4(mfdm_model* m, int it, void* stream) {
   if (rc != MFDM_OK) return rc;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : m->stream;
   if (st != m->stream) MFDM_CU(cudaStreamSynchronize(m->stream));
-  MFDM_CU(mfdm::launch_set_step(m->C, it, st));
   rc = enqueue_step(m, it, st);
   if (rc != MFDM_OK) return rc;
   m->host_step = it + 1;
@@ -1194,7 +1117,7 @@ int mfdm_autotune(mfdm_model* m, int* seg_rows) {
     float best_ms = 0.f;
     for (int variant = 2; variant <= 4; ++variant)
       for (int i = 0; i < n; ++i) {
-        if (variant == 4 && kSegCandidates[i] % 8 != 0) continue;  // tile heights: multiples of 8
+        if (variant == 4 && kSegCandidates[i] % 8 != 0) continue;  // whole multiples of the tile's row step
         float ms = 0.f;
         if ((rc = time_segment_rows(m, kSegCandidates[i], variant, &ms)) != MFDM_OK) return rc;
         if (best.first == 0 || ms < best_ms) {
@@ -1217,7 +1140,7 @@ int mfdm_autotune(mfdm_model* m, int* seg_rows) {
 int mfdm_set_blocks_per_sm(mfdm_model* m, int blocks) {
   if (!m) return fail(MFDM_ERR_ARG, "null handle");
   if (blocks != 0 && blocks != 2 && blocks != 3 && blocks != 4)
-    return fail(MFDM_ERR_ARG, "stage build must be 2, 3 (blocks per SM), 4 (tiles) or 0 (the default)");
+    return fail(MFDM_ERR_ARG, "stage build must be 2, 3, 4 or 0 (the default)");
   DeviceGuard g(m->device);
   MFDM_CU(cudaStreamSynchronize(m->stream));
   m->C.variant = blocks;
@@ -1262,9 +1185,10 @@ int group_enqueue(mfdm_group* g, int k, bool graph) {
     mfdm_model* m = g->ms[i];
     MFDM_CU(cudaStreamWaitEvent(m->stream, g->fork, 0));
     for (int j = 0; j < k; ++j) {
-      const int rc = enqueue_step(m, graph ? j : m->host_step + j, m->stream);
+      const int rc = enqueue_step(m, graph ? j : m->host_step + j, m->stream, nullptr, graph);
       if (rc != MFDM_OK) return rc;
     }
+    if (graph) MFDM_CU(mfdm::launch_advance_step(m->C, k, m->stream));
     MFDM_CU(cudaEventRecord(g->join[i], m->stream));
     MFDM_CU(cudaStreamWaitEvent(g->stream, g->join[i], 0));
   }
@@ -1313,8 +1237,11 @@ int group_run(mfdm_group* g, int nsteps) {
       bool stale = !g->graph;
       for (size_t i = 0; i < g->ms.size() && !stale; ++i) stale = g->gens[i] != g->ms[i]->gen;
       if (stale && (rc = group_capture(g)) != MFDM_OK) return rc;
+      for (mfdm_model* m : g->ms)
+        if ((rc = sync_step(m, g->stream)) != MFDM_OK) return rc;
       MFDM_CU(cudaGraphLaunch(g->graph, g->stream));
       k = kGraphSteps;
+      for (mfdm_model* m : g->ms) m->dev_step += k;
     } else if ((rc = group_enqueue(g, 1, false)) != MFDM_OK) {
       return rc;
     }
@@ -1492,15 +1419,10 @@ int adjoint_build(mfdm_model* m) {
   C.src_pos = nullptr;
   const int stage = 2;  // the third stage: out = U^n + c k, with U^n = 0, and no accumulator
   const float cc = C.rk_c[stage], scale = 1.0f / cc;
-  mfdm::StageMaps maps;
-  maps.fin = m->fst[1]; maps.sin = m->sst[1];
-  maps.fun = m->fpw[2]; maps.sun = m->spw[2];
-  maps.facc = m->fpw[3]; maps.sacc = m->spw[3];
-  maps.fcoef = m->fco; maps.scoef = m->sco;
   const Fields &Out = m->S[0], &In = m->S[1], &Un = m->S[2], &Acc = m->S[3];
   // cells a stage updates: with input 0 and U^n = 1 the output is 1 exactly there
   MFDM_CU(mfdm::adj::fill(Un.fvx, n, 1.0f, st));
-  MFDM_CU(mfdm::launch_stage(C, In, Out, Un, Acc, maps, stage, mfdm::kDirF, st));
+  MFDM_CU(mfdm::launch_stage(C, In, Out, Un, Acc, stage, mfdm::kDirF, st));
   MFDM_CU(mfdm::adj::make_mask(Out.fvx, a->mask, n, st));
   MFDM_CU(cudaMemsetAsync(Un.fvx, 0, size_t(n) * sizeof(float), st));
   MFDM_CU(cudaMemsetAsync(Out.fvx, 0, size_t(n) * sizeof(float), st));
@@ -1533,7 +1455,7 @@ int adjoint_build(mfdm_model* m) {
         for (int cz = 0; cz < 7; ++cz)
           for (int cx = 0; cx < 7; ++cx) {
             MFDM_CU(mfdm::adj::set_lattice(In.fvx, L, arr, cz, cx, 1.0f, st));
-            MFDM_CU(mfdm::launch_stage(C, In, Out, Un, Acc, maps, stage, d, st));
+            MFDM_CU(mfdm::launch_stage(C, In, Out, Un, Acc, stage, d, st));
             MFDM_CU(mfdm::adj::extract(Out.fvx, L, arr, cz, cx, scale, count,
                                        pass ? A.rowptr : nullptr, cursor, A.col, A.val, err, st));
             MFDM_CU(mfdm::adj::set_lattice(In.fvx, L, arr, cz, cx, 0.0f, st));
@@ -1645,63 +1567,27 @@ double* grad_array(mfdm_model* m, int k) {
   return m->adj->grad + (k < 2 ? size_t(k) * nf : 2 * nf + size_t(k - 2) * ns);
 }
 
-// Encodes the TMA maps of the first `nslots` step slots of the slot buffer at
-// `base` into `t` (once per buffer).
-int slot_maps(mfdm_model* m, AdjointState::SlotTable& t, const float* base, size_t nslots) {
-  if (t.base == base && t.maps.size() >= nslots) return MFDM_OK;
-  const mfdm::SetLayout& L = m->adj->L;
-  const size_t len = size_t(L.len);
-  const int P = m->P, nzf = m->cfg.nzf, nzs = m->cfg.nzs;
-  t.base = nullptr;
-  t.maps.assign(nslots, AdjointState::SlotMaps{});
-  int rc;
-  for (size_t j = 0; j < nslots; ++j) {
-    AdjointState::SlotMaps& M = t.maps[j];
-    for (int s = 0; s < 4; ++s) {
-      const float* set = base + (j * 4 + size_t(s)) * len;
-      if ((rc = encode_block(&M.fst[s], set + L.off[0], P, nzf, 3, mfdm::kStageSW, true, m->nshots, m->region)) ||
-          (rc = encode_block(&M.sst[s], set + L.off[3], P, nzs, 5, mfdm::kStageSW, true, m->nshots, m->region)))
-        return rc;
-    }
-    const float* y1 = base + j * 4 * len;
-    if ((rc = encode_block(&M.fun, y1 + L.off[0], P, nzf, 3, mfdm::kStageTX, false, m->nshots, m->region)) ||
-        (rc = encode_block(&M.sun, y1 + L.off[3], P, nzs, 5, mfdm::kStageTX, false, m->nshots, m->region)))
-      return rc;
-  }
-  t.base = base;
-  return MFDM_OK;
-}
-
-// One step run in place in slot j of a slot buffer (maps `t`): stage 0 reads
+// One step run in place in slot j of the slot buffer at `base`: stage 0 reads
 // U^n from the slot's first set, stages 0-2 write the next three sets (the
 // stage inputs the backward pass reads), the last stage writes U^{n+1} into the
 // next slot's first set, or into the handle's state U after the run's last step.
-int enqueue_slot_step(mfdm_model* m, int it, const AdjointState::SlotTable& t, size_t j,
-                      bool last_of_run, cudaStream_t st) {
+int enqueue_slot_step(mfdm_model* m, int it, float* base, size_t j, bool last_of_run,
+                      cudaStream_t st) {
   AdjointState* a = m->adj;
   const mfdm::SetLayout& L = a->L;
   const size_t len = size_t(L.len);
-  float* base = const_cast<float*>(t.base);
   const int d0 = (it & 1) ? mfdm::kDirB : mfdm::kDirF, d1 = 1 - d0;
   const int dir[4] = {d0, d1, d0, d1};
   Fields Y[4];
   for (int s = 0; s < 4; ++s) Y[s] = fields_at(L, base + (j * 4 + size_t(s)) * len);
   const Fields next = last_of_run ? m->S[0] : fields_at(L, base + (j + 1) * 4 * len);
-  const AdjointState::SlotMaps& M = t.maps[j];
   const Fields& Acc = m->S[3];
+  Coef C = m->C;
+  C.step = nullptr;
+  C.it_off = it;
   for (int s = 0; s < 4; ++s) {
-    mfdm::StageMaps maps;
-    maps.fin = M.fst[s];
-    maps.sin = M.sst[s];
-    maps.fun = M.fun;
-    maps.sun = M.sun;
-    maps.facc = m->fpw[3];
-    maps.sacc = m->spw[3];
-    maps.fcoef = m->fco;
-    maps.scoef = m->sco;
-    MFDM_CU(mfdm::launch_stage(m->C, Y[s], s < 3 ? Y[s + 1] : next, Y[0], Acc, maps, s, dir[s], st));
+    MFDM_CU(mfdm::launch_stage(C, Y[s], s < 3 ? Y[s + 1] : next, Y[0], Acc, s, dir[s], st));
   }
-  MFDM_CU(mfdm::launch_finish(m->C, next, st));
   return MFDM_OK;
 }
 
@@ -1827,8 +1713,6 @@ int mfdm_adjoint_forward(mfdm_model* m, int nsteps, int ckpt_every) {
     // strips) must read 0, as in the handle's own sets
     MFDM_CU(cudaMemset(a->keep, 0, nkeep * seg_floats * sizeof(float)));
   }
-  if (nkeep > 0 && (rc = slot_maps(m, a->keep_tab, a->keep, nkeep * size_t(ckpt_every))) != MFDM_OK)
-    return rc;
   a->nkeep = int(nkeep);
   a->nsteps = -1;
   if ((rc = clear_state(m)) != MFDM_OK) return rc;
@@ -1844,7 +1728,7 @@ int mfdm_adjoint_forward(mfdm_model* m, int nsteps, int ckpt_every) {
                                 cudaMemcpyDeviceToDevice, m->stream));
       for (int j = 0; j < todo; ++j) {
         const bool last = k + 1 == ncp && j + 1 == todo;
-        if ((rc = enqueue_slot_step(m, m->host_step, a->keep_tab, j0 + size_t(j), last, m->stream)) !=
+        if ((rc = enqueue_slot_step(m, m->host_step, a->keep, j0 + size_t(j), last, m->stream)) !=
             MFDM_OK)
           return rc;
         ++m->host_step;
@@ -1906,8 +1790,6 @@ int mfdm_adjoint_backward(mfdm_model* m, const float* res_svx, const float* res_
     MFDM_CU(cudaMemset(a->seg, 0, size_t(inner) * 4 * len * sizeof(float)));
     a->seg_steps = size_t(inner);
   }
-  if (a->nkeep < ncp && (rc = slot_maps(m, a->seg_tab[0], a->seg, a->seg_steps)) != MFDM_OK)
-    return rc;
   if (a->nkeep < ncp && inner < every && ninner > a->inner_sets) {
     cudaFree(a->inner);
     a->inner = nullptr;
@@ -1939,7 +1821,6 @@ int mfdm_adjoint_backward(mfdm_model* m, const float* res_svx, const float* res_
       MFDM_CU(cudaMemset(a->seg2, 0, a->seg_steps * 4 * len * sizeof(float)));
     }
   }
-  if (dbl && (rc = slot_maps(m, a->seg_tab[1], a->seg2, a->seg_steps)) != MFDM_OK) return rc;
   auto buf_of = [&](int k) { return (dbl && (k & 1)) ? 1 : 0; };
   auto buf_ptr = [&](int b) { return b ? a->seg2 : a->seg; };
   // restore checkpoint k into the first slot of buffer b and recompute steps
@@ -1948,10 +1829,9 @@ int mfdm_adjoint_backward(mfdm_model* m, const float* res_svx, const float* res_
     MFDM_CU(cudaStreamWaitEvent(st, a->ev_rev[b], 0));
     MFDM_CU(cudaMemcpyAsync(buf_ptr(b), from_ckpt ? a->ckpt + size_t(k) * len : from,
                             len * sizeof(float), cudaMemcpyDeviceToDevice, st));
-    MFDM_CU(mfdm::launch_set_step(m->C, u0, st));
     for (int n = u0; n < u1; ++n) {
       int rc2;
-      if ((rc2 = enqueue_slot_step(m, n, a->seg_tab[b], size_t(n - u0), n + 1 == u1, st)) != MFDM_OK)
+      if ((rc2 = enqueue_slot_step(m, n, buf_ptr(b), size_t(n - u0), n + 1 == u1, st)) != MFDM_OK)
         return rc2;
     }
     MFDM_CU(cudaEventRecord(a->ev_seg[b], st));
@@ -1980,7 +1860,6 @@ int mfdm_adjoint_backward(mfdm_model* m, const float* res_svx, const float* res_
       MFDM_CU(cudaStreamWaitEvent(st, a->ev_rev[0], 0));
       MFDM_CU(cudaMemcpyAsync(m->S[0].fvx, a->ckpt + size_t(k) * len, len * sizeof(float),
                               cudaMemcpyDeviceToDevice, st));
-      MFDM_CU(mfdm::launch_set_step(m->C, t0, st));
       m->host_step = t0;
       for (int i = 0; t0 + i * inner < t1; ++i) {
         MFDM_CU(cudaMemcpyAsync(a->inner + size_t(i) * len, m->S[0].fvx, len * sizeof(float),
@@ -2361,10 +2240,9 @@ int solid_build(mfdm_solid* m, const SolidHost& h, int device) {
   C.step = misc;
   C.done = reinterpret_cast<unsigned*>(misc + 1);
   C.status = misc + 2;
-  // RK4 weights formed in float like the reference (src/pml_fs_kernels.cu:95-380)
-  const float dt = p.dt;
-  C.rk_c[0] = dt / 2; C.rk_c[1] = dt / 2; C.rk_c[2] = dt; C.rk_c[3] = dt / 6;
-  C.rk_w[0] = dt / 6; C.rk_w[1] = dt / 3; C.rk_w[2] = dt / 3;
+  const mfdm::RkOnce once = mfdm::rk_once(p.dt);
+  C.rk_c[0] = p.dt / 2; C.rk_c[1] = p.dt / 2; C.rk_c[2] = p.dt; C.rk_c[3] = once.c;
+  C.rk_w = once.w;
   C.gap = m->gap;
   C.srcx = m->srcx.empty() ? -1 : m->srcx[0];
   C.srcz = m->srcx.empty() ? 0 : m->srcz[0];

@@ -18,7 +18,7 @@
 // The Ricker and PML values come from the same host functions as the handle
 // path's (mfdm::ricker_ref, mfdm::pml_cell), so both entry points step with
 // bit-identical tables. The first call on a device caches the array's address
-// and configures the kernels there; after cudaDeviceReset of that device the
+// there; after cudaDeviceReset of that device the
 // cache is stale, so a process that resets a device must not call this entry
 // point on it again.
 #include <cuda_runtime.h>
@@ -44,12 +44,6 @@ struct DeviceSlot {
 DeviceSlot g_slots[kMaxDevices];
 std::mutex g_setup_mutex;
 
-// 5x5 source weights (src/elements.cu:34-40) and the interface filter (src/elements.cu:30-33).
-const float kSrcW[25] = {0.0030f, 0.0133f, 0.0219f, 0.0133f, 0.0030f, 0.0133f, 0.0596f,
-                         0.0983f, 0.0596f, 0.0133f, 0.0219f, 0.0983f, 0.1621f, 0.0983f,
-                         0.0219f, 0.0133f, 0.0596f, 0.0983f, 0.0596f, 0.0133f, 0.0030f,
-                         0.0133f, 0.0219f, 0.0133f, 0.0030f};
-const float kW7[7] = {1.1e-13f, 1.678e-06f, 0.03419f, 0.93163f, 0.03419f, 1.678e-06f, 1.1e-13f};
 
 int err(int code, const char* msg) { return mfdm::set_error(code, msg); }
 
@@ -60,7 +54,7 @@ int err(int code, const char* msg) { return mfdm::set_error(code, msg); }
   } while (0)
 
 // The first call on a device resolves the array's device address (host code
-// cannot use the symbol itself) and configures the kernels on that device.
+// cannot use the symbol itself).
 int setup_device(unsigned char** base) {
   int dev = -1;
   NA_CU(cudaGetDevice(&dev));
@@ -71,8 +65,6 @@ int setup_device(unsigned char** base) {
     void* p = nullptr;
     NA_CU(cudaGetSymbolAddress(&p, g_noalloc_scratch));
     if (!p) return err(MFDM_ERR_CUDA, "no device address for the static scratch array");
-    NA_CU(mfdm::configure_device());
-    NA_CU(mfdm::upload_constants(kSrcW, kW7));
     s.base = static_cast<unsigned char*>(p);
     s.ready = true;
   }
@@ -128,7 +120,7 @@ extern "C" int mfdm_step_noalloc(const mfdm_device_model* dm, int it, int nsteps
 
   // Layout of the scratch array (the same blocks an open handle allocates).
   const int nz = nzf + nzs - 1;
-  const int P = round_up(nx > mfdm::kStageSW ? nx : mfdm::kStageSW, 32);
+  const int P = round_up(nx > mfdm::kMinPitch ? nx : mfdm::kMinPitch, 32);
   const int Ps = round_up(2 * npd > 1 ? 2 * npd : 1, 4), npdr = npd > 1 ? npd : 1;
   size_t off = 0;
   auto take = [&](size_t nfloats) {
@@ -141,7 +133,7 @@ extern "C" int mfdm_step_noalloc(const mfdm_device_model* dm, int it, int nsteps
   size_t o_met[5];
   for (int q = 0; q < 5; ++q) o_met[q] = take(ng);
   const size_t o_pmlx = take(size_t(nx) * 4), o_pmlz = take(size_t(nzs) * 4),
-               o_nrm = take(size_t(nx) * 2), o_ipre = take(size_t(8) * P), o_misc = take(64),
+               o_nrm = take(size_t(nx) * 2), o_spare = take(size_t(8) * P), o_misc = take(64),
                o_amp = take(size_t(kAmpSteps) * 4);
   size_t o_fb[4], o_sb[4], o_ade[4][12];
   for (int s = 0; s < 4; ++s) {
@@ -154,6 +146,7 @@ extern "C" int mfdm_step_noalloc(const mfdm_device_model* dm, int it, int nsteps
     for (int q = 0; q < 4; ++q) o_ade[s][4 + q] = take(size_t(nzs) * Ps);
     for (int q = 0; q < 4; ++q) o_ade[s][8 + q] = take(size_t(npdr) * P);
   }
+  (void)o_spare;  // the size that decides which models fit stays as it was
   if (off > kNoAllocBytes) {
     char msg[200];
     snprintf(msg, sizeof msg,
@@ -258,26 +251,10 @@ extern "C" int mfdm_step_noalloc(const mfdm_device_model* dm, int it, int nsteps
   C.gap = 1;
   C.rec = nullptr;  // receivers: the caller reads its own state arrays
   C.rec_cap = 0;
-  C.ipre = F(o_ipre);
   int* misc = reinterpret_cast<int*>(F(o_misc));
-  C.step = misc;
-  C.done = reinterpret_cast<unsigned*>(misc + 1);
+  C.step = nullptr;  // every launch carries its own time index (it_off)
   C.status = misc + 2;
 
-  CUtensorMap fst[4], sst[4], fpw[4], spw[4], fcm, scm;
-  for (int s = 0; s < 4; ++s) {
-    // state maps: one shot (the kernels address the shot as a fourth coordinate)
-    if ((rc = mfdm::encode_block_map(&fst[s], F(o_fb[s]), P, nzf, 3, mfdm::kStageSW, true, 1, 256)) ||
-        (rc = mfdm::encode_block_map(&sst[s], F(o_sb[s]), P, nzs, 5, mfdm::kStageSW, true, 1, 256)) ||
-        (rc = mfdm::encode_block_map(&fpw[s], F(o_fb[s]), P, nzf, 3, mfdm::kStageTX, false, 1, 256)) ||
-        (rc = mfdm::encode_block_map(&spw[s], F(o_sb[s]), P, nzs, 5, mfdm::kStageTX, false, 1, 256)))
-      return rc;
-  }
-  if ((rc = mfdm::encode_block_map(&fcm, fco, P, nzf, 6, mfdm::kStageTX, false)) ||
-      (rc = mfdm::encode_block_map(&scm, sco, P, nzs, 9, mfdm::kStageTX, false)))
-    return rc;
-
-  NA_CU(mfdm::launch_set_step(C, it, st));
   const int in_set[4] = {0, 1, 2, 1}, out_set[4] = {1, 2, 1, 0};
   const float half = float(double(dt) * 0.5);
   for (int k0 = 0; k0 < nsteps; k0 += kAmpSteps) {
@@ -301,19 +278,10 @@ extern "C" int mfdm_step_noalloc(const mfdm_device_model* dm, int it, int nsteps
     for (int k = k0; k < k0 + nk; ++k) {
       const int d0 = ((it + k) & 1) ? mfdm::kDirB : mfdm::kDirF, d1 = 1 - d0;
       const int dir[4] = {d0, d1, d0, d1};
+      C.it_off = it + k;
       for (int s = 0; s < 4; ++s) {
-        mfdm::StageMaps maps;
-        maps.fin = fst[in_set[s]];
-        maps.sin = sst[in_set[s]];
-        maps.fun = fpw[0];
-        maps.sun = spw[0];
-        maps.facc = fpw[3];
-        maps.sacc = spw[3];
-        maps.fcoef = fcm;
-        maps.scoef = scm;
-        NA_CU(mfdm::launch_stage(C, S[in_set[s]], S[out_set[s]], S[0], S[3], maps, s, dir[s], st));
+        NA_CU(mfdm::launch_stage(C, S[in_set[s]], S[out_set[s]], S[0], S[3], s, dir[s], st));
       }
-      NA_CU(mfdm::launch_finish(C, S[0], st));
     }
   }
   // The wavefield out.
@@ -323,8 +291,6 @@ extern "C" int mfdm_step_noalloc(const mfdm_device_model* dm, int it, int nsteps
   int status = 0;
   NA_CU(cudaMemcpyAsync(&status, C.status, sizeof(int), cudaMemcpyDeviceToHost, st));
   NA_CU(cudaStreamSynchronize(st));
-  if (status & 2)
-    return err(MFDM_ERR_CUDA, "a stage kernel pipeline wait timed out; the state arrays are undefined");
-  if (status & 1) return err(MFDM_ERR_NONFINITE, "non-finite values reached the interface rows");
+  if (status) return err(MFDM_ERR_NONFINITE, "non-finite values reached the interface rows");
   return MFDM_OK;
 }

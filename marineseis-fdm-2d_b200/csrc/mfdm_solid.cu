@@ -387,7 +387,7 @@ template <int DIR, int KIND>
 cudaError_t launch_t(const SCoef& C, const SFields& in, const SFields& out, const SFields& un,
                      const SFields& acc, int s, cudaStream_t st) {
   const dim3 grid(unsigned((C.nx - 6 + kBX - 1) / kBX), unsigned((C.nz - 6 + kTZ - 1) / kTZ));
-  const float c = C.rk_c[s], w = KIND == kStageSecond ? C.rk_w[s] : 0.f;
+  const float c = C.rk_c[s], w = KIND == kStageSecond ? C.rk_w : 0.f;
   if (C.cpml)
     k_stage<DIR, KIND, true><<<grid, dim3(kBX, kBY), 0, st>>>(C, in, out, un, acc, s, c, w);
   else

@@ -28,8 +28,8 @@ struct SCoef {
   const float* __restrict__ src_amp;  // Ricker value per (step, stage): [steps][4]
   int src_steps;
   int srcx, srcz;                   // source cell (srcx < 0: none)
-  float rk_c[4];                    // dt/2, dt/2, dt, dt/6
-  float rk_w[3];                    // dt/6, dt/3, dt/3
+  float rk_c[4];                    // dt/2, dt/2, dt and k4's weight (rk_once)
+  float rk_w;                       // k2's weight (rk_once)
   int gap, rec_cap;
   float* rec;                       // [rec_cap][nx]: solid vz on row rec_row
   int rec_row;                      // 3 (free surface) or 30 (cpml), src/main.cu:303-311

@@ -1,7 +1,7 @@
-"""The RK4 bookkeeping of the stage kernels (mfdm_device.cuh, rk_acc / rk_last), restated in numpy float32.
+"""The once-a-step RK4 bookkeeping (mfdm_device.cuh, rk_acc / rk_last / rk_once), restated in numpy float32.
 
-A step accumulates once, in the second stage: acc = 2/3 U + (Y2 - U)/3 + dt/3 k2, and
-U' = acc + Y4/3 + dt/6 k4. The weights come from the header, so they are checked as compiled.
+A step accumulates once, in the second stage: acc = 2/3 U + (Y2 - U)/3 + w k2, and
+U' = acc + Y4/3 + c k4, w and c close to dt/3 and dt/6 (rk_once). The weights come from the header, so they are checked as compiled.
 """
 import os
 import re
@@ -66,8 +66,10 @@ def test_the_step_is_classical_rk4(z):
     y2 = fma(dt / F(2), k1, u)
     k2 = lam * y2
     y3 = fma(dt / F(2), k2, u)
-    acc = rk_acc(k2, y2, u, dt / F(3))
+    c = F(0.5 * float(W) * float(dt))
+    w = F(float(dt) - 1.5 * float(W) * float(dt) - float(c))
+    acc = rk_acc(k2, y2, u, w)
     y4 = fma(dt, lam * y3, u)
-    got = rk_last(lam * y4, y4, acc, dt / F(6)).astype(np.float64)
+    got = rk_last(lam * y4, y4, acc, c).astype(np.float64)
     want = u.astype(np.float64) * (1 + zz + zz ** 2 / 2 + zz ** 3 / 6 + zz ** 4 / 24)
     assert np.max(np.abs(got / want - 1)) <= 4 * 2.0 ** -24 * (1 + 4 * abs(zz))
