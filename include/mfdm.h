@@ -402,8 +402,8 @@ int mfdm_dispersion_velocities(double c_min, double c_max, double dc);
 /* gather: host [nt][ntr] float32 (the mfdm_get_records layout, traces already
  * selected); offsets: host [ntr] signed source-receiver offsets (m); fs:
  * sampling rate (Hz); amplitude: host [nt/2+1][nv] with nv from
- * mfdm_dispersion_velocities. Allocates its device buffers on `device` and
- * frees them before it returns. */
+ * mfdm_dispersion_velocities. Its device buffers on `device` come from a memory
+ * pool of the library, which keeps at most 64 MiB of them between calls. */
 int mfdm_dispersion_image(const float* gather, int nt, int ntr, const double* offsets, double fs,
                           double c_min, double c_max, double dc, float* amplitude, int device);
 
