@@ -1925,6 +1925,8 @@ struct mfdm_solid {
   int nt = 0, snapshot = 1, gap = 1;
   std::vector<int> srcx, srcz;
   int isrc = 0, host_step = 0;
+  int dev_step = 0;  // the device step counter's value once the stream gets there
+  int* d_srcpos = nullptr;  // source cell (x, z; x < 0: none)
   char* dmem = nullptr;
   size_t dbytes = 0;
   mfdm::solid::SFields S[4];  // U, stage A, stage B, accumulator
@@ -2056,15 +2058,18 @@ int solid_capacity(mfdm_solid* m, int steps) {
   return MFDM_OK;
 }
 
-int solid_enqueue_step(mfdm_solid* m, int it, cudaStream_t st) {
+// Enqueues one step of time index `it` (captured: the device step counter + it).
+int solid_enqueue_step(mfdm_solid* m, int it, cudaStream_t st, bool captured = false) {
+  mfdm::solid::SCoef C = m->C;
+  if (!captured) C.step = nullptr;
+  C.it_off = it;
   const int d0 = (it & 1) ? mfdm::kDirB : mfdm::kDirF, d1 = 1 - d0;
   const mfdm::solid::SFields &U = m->S[0], &A = m->S[1], &B = m->S[2], &Acc = m->S[3];
   const mfdm::solid::SFields* in[4] = {&U, &A, &B, &A};
   const mfdm::solid::SFields* out[4] = {&A, &B, &A, &U};
   const int dir[4] = {d0, d1, d0, d1};
   for (int s = 0; s < 4; ++s)
-    MFDM_CU(mfdm::solid::launch_stage(m->C, *in[s], *out[s], U, Acc, s, dir[s], st));
-  MFDM_CU(mfdm::solid::launch_finish(m->C, U, st));
+    MFDM_CU(mfdm::solid::launch_stage(C, *in[s], *out[s], U, Acc, s, dir[s], st));
   return MFDM_OK;
 }
 
@@ -2076,7 +2081,9 @@ int solid_enqueue_steps(mfdm_solid* m, int nsteps) {
         cudaGraph_t g = nullptr;
         MFDM_CU(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
         rc = MFDM_OK;
-        for (int k = 0; k < kGraphSteps && rc == MFDM_OK; ++k) rc = solid_enqueue_step(m, k, m->stream);
+        for (int k = 0; k < kGraphSteps && rc == MFDM_OK; ++k) rc = solid_enqueue_step(m, k, m->stream, true);
+        if (rc == MFDM_OK && mfdm::solid::launch_advance_step(m->C, kGraphSteps, m->stream) != cudaSuccess)
+          rc = fail(MFDM_ERR_CUDA, "graph capture: step counter");
         const cudaError_t e = cudaStreamEndCapture(m->stream, &g);
         if (rc != MFDM_OK) {
           if (g) cudaGraphDestroy(g);
@@ -2088,8 +2095,11 @@ int solid_enqueue_steps(mfdm_solid* m, int nsteps) {
         if (e2 != cudaSuccess)
           return fail(MFDM_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e2));
       }
+      if (m->dev_step != m->host_step)
+        MFDM_CU(mfdm::solid::launch_set_step(m->C, m->host_step, m->stream));
       MFDM_CU(cudaGraphLaunch(m->graph, m->stream));
       m->host_step += kGraphSteps;
+      m->dev_step = m->host_step;
       nsteps -= kGraphSteps;
     } else {
       if ((rc = solid_enqueue_step(m, m->host_step, m->stream)) != MFDM_OK) return rc;
@@ -2097,6 +2107,14 @@ int solid_enqueue_steps(mfdm_solid* m, int nsteps) {
       --nsteps;
     }
   }
+  return MFDM_OK;
+}
+
+// Writes the current source's cell to the device, where the kernels read it.
+int solid_source(mfdm_solid* m) {
+  const int pos[2] = {m->srcx.empty() ? -1 : m->srcx[size_t(m->isrc)],
+                      m->srcx.empty() ? 0 : m->srcz[size_t(m->isrc)]};
+  MFDM_CU(cudaMemcpyAsync(m->d_srcpos, pos, sizeof pos, cudaMemcpyHostToDevice, m->stream));
   return MFDM_OK;
 }
 
@@ -2108,6 +2126,7 @@ int solid_rewind(mfdm_solid* m, bool clear) {
   MFDM_CU(cudaMemsetAsync(m->C.status, 0, sizeof(int), m->stream));
   m->host_step = 0;
   MFDM_CU(mfdm::solid::launch_set_step(m->C, 0, m->stream));
+  m->dev_step = 0;
   MFDM_CU(cudaStreamSynchronize(m->stream));
   return MFDM_OK;
 }
@@ -2238,15 +2257,16 @@ int solid_build(mfdm_solid* m, const SolidHost& h, int device) {
   C.pmlz = reinterpret_cast<const float4*>(F(o_pz));
   int* misc = reinterpret_cast<int*>(F(o_misc));
   C.step = misc;
-  C.done = reinterpret_cast<unsigned*>(misc + 1);
+  C.it_off = 0;
   C.status = misc + 2;
+  m->d_srcpos = misc + 4;
+  C.src_pos = reinterpret_cast<const int2*>(m->d_srcpos);
   const mfdm::RkOnce once = mfdm::rk_once(p.dt);
   C.rk_c[0] = p.dt / 2; C.rk_c[1] = p.dt / 2; C.rk_c[2] = p.dt; C.rk_c[3] = once.c;
   C.rk_w = once.w;
   C.gap = m->gap;
-  C.srcx = m->srcx.empty() ? -1 : m->srcx[0];
-  C.srcz = m->srcx.empty() ? 0 : m->srcz[0];
   int rc;
+  if ((rc = solid_source(m)) != MFDM_OK) return rc;
   if ((rc = solid_capacity(m, std::max(p.nt, 1))) != MFDM_OK) return rc;
   MFDM_CU(cudaStreamSynchronize(m->stream));
   return solid_rewind(m, false);
@@ -2323,9 +2343,8 @@ int mfdm_solid_set_shot(mfdm_solid* m, int isrc, int reset_state) {
     return fail(MFDM_ERR_ARG, "shot index out of range");
   DeviceGuard g(m->device);
   m->isrc = isrc;
-  m->C.srcx = m->srcx.empty() ? -1 : m->srcx[size_t(isrc)];
-  m->C.srcz = m->srcx.empty() ? 0 : m->srcz[size_t(isrc)];
-  solid_release_graph(m);  // the source cell is baked into the kernel arguments
+  const int rc = solid_source(m);
+  if (rc != MFDM_OK) return rc;
   return solid_rewind(m, reset_state != 0);
 }
 

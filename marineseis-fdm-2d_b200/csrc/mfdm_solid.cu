@@ -6,36 +6,32 @@
 // update_stress, which run as two kernels on two streams), the free-surface
 // ghost fluxes (built on the fly from the stage input instead of a separate
 // build_ghost_flux launch), the explosive source and the fused RK4 update
-// (the reference's vector_add / vector_self_add launches over full grids).
-// A fifth launch per step samples the receiver row and advances the device
-// step counter. Each block stages the five stage-input fields of its 32x16
-// cells and their 3-cell halo in shared memory with independent float4 loads
-// (all in flight at once, together with the point-wise operands of every
-// thread's first row), then every thread computes two rows from shared memory;
-// coefficients, ADE memory and the RK operands are point-wise global reads,
-// all of a row's issued before its arithmetic and its stores.
+// (the reference's vector_add / vector_self_add launches over full grids); the
+// last stage also samples the receiver row. Blocks are tiles of 32 columns (as
+// the fluid-solid kernels', mfdm_stage.cu), the slow ones first: 8 rows from the
+// free surface down with the general right-hand side, 8 rows of an absorbing
+// strip, or `tr` interior rows with a branch-free body. Every operand of a cell
+// is loaded before its arithmetic and its stores.
+//
+// Bound: HBM. A step moves 96 floats a cell (inputs 4 x 5, U^n 2 x 5, the
+// accumulator 2 x 5, coefficients 4 x 9, outputs 4 x 5), 250 us of 2048x2048 at
+// the measured copy rate. Measured, us a step, against tiles of 32 x 16 that loaded
+// operand by operand and sampled the receivers in a fifth launch: 400x400 50 -> 23,
+// 1000x1000 122 -> 92, 2048x2048 338 -> 300, 4096x4096 1146 -> 1058.
+#include <algorithm>
+
 #include "mfdm_device.cuh"
 #include "mfdm_solid.h"
+#include "mfdm_tile.cuh"
 
 namespace mfdm {
 namespace solid {
 namespace {
 
-constexpr int kBX = 32, kBY = 8;
-#ifndef MFDM_SOLID_ROWS
-#define MFDM_SOLID_ROWS 16
-#endif
-constexpr int kTZ = MFDM_SOLID_ROWS;  // rows per block (kTZ / kBY per thread)
-static_assert(kTZ % kBY == 0 && 5 * (kTZ + 6) * (kBX + 8) * 4 <= 48 * 1024, "tile rows");
-constexpr int kHW = kBX + 8;     // tile row: columns c0 .. c0 + 39, c0 = first cell - 3
-constexpr int kHH = kTZ + 6;     // tile rows: r0 .. r0 + kTZ + 5, r0 = first row - 3
+using namespace tiles;
+
 enum { kVX = 0, kVZ, kSX, kSZ, kSXZ };
 
-// The 5x5 weights of the explosive source (src/elements.cu:34-40).
-__constant__ float kSrcW[25] = {0.0030f, 0.0133f, 0.0219f, 0.0133f, 0.0030f, 0.0133f, 0.0596f,
-                                0.0983f, 0.0596f, 0.0133f, 0.0219f, 0.0983f, 0.1621f, 0.0983f,
-                                0.0219f, 0.0133f, 0.0596f, 0.0983f, 0.0596f, 0.0133f, 0.0030f,
-                                0.0133f, 0.0219f, 0.0133f, 0.0030f};
 // Point-wise coefficients of a cell, in this order.
 enum { kCXIX = 0, kCXIZ, kCZEX, kCZEZ, kCRR, kC11, kC13, kC33, kC55, kNCoef };
 
@@ -57,21 +53,21 @@ __device__ __forceinline__ int zeta_row(int iz, int nz, int npd) {
 // no free surface, so every row takes the plain biased operators (rows 0..2
 // are zero), and the zeta-PML also covers the top band (rows 3..npd+2).
 // `A(q, dz, dx)` returns stage-input field q (kVX..kSXZ) dz rows and dx columns
-// away, |dz|, |dx| <= 3; the ADE memory of S is read from global memory.
-// IN: the caller guarantees a cell at least three rows below the free surface
-// and outside every absorbing strip (the branch-free body of interior blocks).
-// `K(c)` returns point-wise coefficient c (kCXIX..kC55) of the cell.
-template <int DIR, bool IN, bool CPML, class Acc, class Kc>
-__device__ __forceinline__ Out rhs(const SCoef& C, const SFields& S, const Acc& A, const Kc& K,
-                                   int iz, int ix) {
+// away, |dz|, |dx| <= 3; `K(c)` point-wise coefficient c (kCXIX..kC55).
+// SURF: the cell may be one of the three rows under the free surface. PML: it may
+// lie in the xi strips (`side`, ADE memory xa, factors px) or in a zeta band
+// (`bottom`, za, pz).
+template <int DIR, bool SURF, bool PML, bool CPML, class Acc, class Kc>
+__device__ __forceinline__ Out rhs(const SCoef& C, const Acc& A, const Kc& K, int iz, int ix,
+                                   bool side, bool bottom, const float* xa, const float* za,
+                                   float4 px, float4 pz) {
   Out o;
-  const int P = C.P, nx = C.nx, nz = C.nz, npd = C.npd;
+  const int P = C.P;
   const size_t i = (size_t)iz * P + ix;
-  const int dist = (IN || CPML) ? 3 : iz - 3, distx = min(ix - 3, nx - 4 - ix);
-  const bool side = !IN && distx < npd;
-  const bool bottom = !IN && (iz >= nz - 3 - npd || (CPML && iz <= npd + 2));
-  const int scol = side ? xstrip_col(ix, nx, npd) : 0;
-  const size_t si = (size_t)iz * C.Ps + scol, zi = (size_t)zeta_row<CPML>(iz, nz, npd) * P + ix;
+  const int dist = SURF && !CPML ? iz - 3 : 3;
+  constexpr bool IN = !SURF;
+  side = PML && side;
+  bottom = PML && bottom;
   const float xix = K(kCXIX), xiz = K(kCXIZ), zex = K(kCZEX), zez = K(kCZEZ);
   const float gxixi = xix * xix + xiz * xiz, gzeze = zex * zex + zez * zez;
   const float gxize = xix * zex + xiz * zez;
@@ -133,16 +129,16 @@ __device__ __forceinline__ Out rhs(const SCoef& C, const SFields& S, const Acc& 
     o.vx = rvx * ir;
     o.vz = rvz * ir;
     if (side) {
-      const float4 p = __ldg(C.pmlx + ix);
-      const float V0 = __ldg(S.x[0] + si), V1 = __ldg(S.x[1] + si);
+      const float4 p = px;
+      const float V0 = xa[0], V1 = xa[1];
       o.XV0 = -p.y * V0 + p.x * dxx;
       o.XV1 = -p.y * V1 + p.x * dxz;
       o.vx += ((p.z - 1.0f) * dxx - p.z * V0) * ir;
       o.vz += ((p.z - 1.0f) * dxz - p.z * V1) * ir;
     }
     if (bottom) {
-      const float4 p = __ldg(C.pmlz + iz);
-      const float V0 = __ldg(S.z[0] + zi), V1 = __ldg(S.z[1] + zi);
+      const float4 p = pz;
+      const float V0 = za[0], V1 = za[1];
       o.ZV0 = -p.y * V0 + p.x * dzx;
       o.ZV1 = -p.y * V1 + p.x * dzz;
       o.vx += ((p.z - 1.0f) * dzx - p.z * V0) * ir;
@@ -163,8 +159,8 @@ __device__ __forceinline__ Out rhs(const SCoef& C, const SFields& S, const Acc& 
       o.sz = (c13 * a0 + c33 * a1) * dvx_dxi + (c13 * a3 + c33 * a4) * dvz_dxi;
       o.sxz = c55 * (a2 * dvx_dxi + a5 * dvz_dxi);
       if (side) {
-        const float4 p = __ldg(C.pmlx + ix);
-        const float E0 = __ldg(S.x[2] + si), E1 = __ldg(S.x[3] + si);
+        const float4 p = px;
+        const float E0 = xa[2], E1 = xa[3];
         o.XE0 = -p.y * E0 + p.x * dvx_dxi;
         o.XE1 = -p.y * E1 + p.x * dvz_dxi;
         const float cxx_x = c11 * a0 + c13 * a1, cxx_z = c11 * a3 + c13 * a4;
@@ -181,8 +177,8 @@ __device__ __forceinline__ Out rhs(const SCoef& C, const SFields& S, const Acc& 
     o.sxz = c55 * (xiz * dvx_dxi + zez * dvx_dze + xix * dvz_dxi + zex * dvz_dze);
     if (side) {
       const float Dvx = dvx_dxi + (gxize / gxixi) * dvx_dze, Dvz = dvz_dxi + (gxize / gxixi) * dvz_dze;
-      const float4 p = __ldg(C.pmlx + ix);
-      const float E0 = __ldg(S.x[2] + si), E1 = __ldg(S.x[3] + si), invb = p.z;
+      const float4 p = px;
+      const float E0 = xa[2], E1 = xa[3], invb = p.z;
       o.XE0 = -p.y * E0 + p.x * Dvx;
       o.XE1 = -p.y * E1 + p.x * Dvz;
       o.sx += c11 * (invb - 1.0f) * xix * Dvx + c13 * (invb - 1.0f) * xiz * Dvz -
@@ -194,8 +190,8 @@ __device__ __forceinline__ Out rhs(const SCoef& C, const SFields& S, const Acc& 
     }
     if (bottom) {
       const float Dvx = dvx_dze + (gxize / gzeze) * dvx_dxi, Dvz = dvz_dze + (gxize / gzeze) * dvz_dxi;
-      const float4 p = __ldg(C.pmlz + iz);
-      const float E0 = __ldg(S.z[2] + zi), E1 = __ldg(S.z[3] + zi), invb = p.z;
+      const float4 p = pz;
+      const float E0 = za[2], E1 = za[3], invb = p.z;
       o.ZE0 = -p.y * E0 + p.x * Dvx;
       o.ZE1 = -p.y * E1 + p.x * Dvz;
       o.sx += c11 * (invb - 1.0f) * zex * Dvx + c13 * (invb - 1.0f) * zez * Dvz -
@@ -209,31 +205,18 @@ __device__ __forceinline__ Out rhs(const SCoef& C, const SFields& S, const Acc& 
   return o;
 }
 
-template <int KIND>
-__device__ __forceinline__ void upd(float k, const float* in, const float* un, float* out,
-                                    float* acc, size_t i, float c, float w) {
-  rk_update<KIND>(k, KIND == kStageThird ? 0.f : __ldg(in + i), un, out, acc, i, c, w);
-}
-
 // The point-wise operands of one cell: U^n or, in the last stage, the
-// accumulator (`u`) and the coefficients (`k`). They are loaded into registers before any store of the row -- the
-// first row's before the tile barrier, so that their DRAM round trips overlap
-// the tile load (the output and accumulator pointers may alias the inputs as
-// far as the compiler knows, which would otherwise order each field's loads
-// after the previous field's stores). Loading the next row's under the
-// current row's arithmetic needs 80 registers and was slower.
+// accumulator (`u`) and the coefficients (`k`).
 struct Pt { float u[5], k[kNCoef]; };
 
 template <int KIND>
 __device__ __forceinline__ void load_pt(Pt& p, const SCoef& C, const SFields& un,
                                         const SFields& acc, size_t i) {
-  const float* const pu[5] = {un.vx, un.vz, un.sx, un.sz, un.sxz};
-  const float* const pa[5] = {acc.vx, acc.vz, acc.sx, acc.sz, acc.sxz};
+  const float* const pu = KIND == kStageLast ? acc.vx : un.vx;
+  const size_t n = (size_t)C.nz * C.P;  // the five fields lie one after another
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    if (KIND == kStageSecond || KIND == kStageThird) p.u[q] = __ldg(pu[q] + i);
-    if (KIND == kStageLast) p.u[q] = pa[q][i];
-  }
+  for (int q = 0; q < 5; ++q)
+    if (KIND != kStageFirst) p.u[q] = __ldg(pu + q * n + i);
   p.k[kCXIX] = __ldg(C.xix + i);
   p.k[kCXIZ] = __ldg(C.xiz + i);
   p.k[kCZEX] = __ldg(C.zex + i);
@@ -245,179 +228,209 @@ __device__ __forceinline__ void load_pt(Pt& p, const SCoef& C, const SFields& un
   p.k[kC55] = __ldg(C.C55 + i);
 }
 
-// y(q): the stage input's field q at the cell.
-template <int KIND, class Y>
-__device__ __forceinline__ void store5(const Out& o, const Pt& r, const Y& y, const SFields& out,
-                                       const SFields& acc, size_t i, float c, float w) {
-  float* const po[5] = {out.vx, out.vz, out.sx, out.sz, out.sxz};
-  float* const pa[5] = {acc.vx, acc.vz, acc.sx, acc.sz, acc.sxz};
-  const float k[5] = {o.vx, o.vz, o.sx, o.sz, o.sxz};
+// The four ADE values of a strip cell: the stage input's (`y`) and U^n's or the
+// accumulator's (`u`).
+template <int KIND>
+__device__ __forceinline__ void load_ade(float* y, float* u, float* const* in, float* const* un,
+                                         float* const* acc, size_t i) {
 #pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    if (KIND == kStageFirst) {
-      po[q][i] = fmaf(c, k[q], y(q));
-    } else if (KIND == kStageLast) {
-      po[q][i] = rk_last(k[q], y(q), r.u[q], c);
-    } else {
-      po[q][i] = fmaf(c, k[q], r.u[q]);
-      if (KIND == kStageSecond) pa[q][i] = rk_acc(k[q], y(q), r.u[q], w);
-    }
+  for (int q = 0; q < 4; ++q) {
+    y[q] = __ldg(in[q] + i);
+    if (KIND == kStageSecond || KIND == kStageThird) u[q] = __ldg(un[q] + i);
+    if (KIND == kStageLast) u[q] = __ldg(acc[q] + i);
   }
 }
 
-// The kTZ / kBY rows of column ix owned by this thread, from the staged tile;
-// `p` holds the first row's point-wise operands on entry.
-template <int DIR, int KIND, bool IN, bool CPML>
-__device__ __forceinline__ void rows(const SCoef& C, const SFields& in, const SFields& out,
-                                     const SFields& un, const SFields& acc,
-                                     const float (&tile)[5][kHH][kHW], int r0, int ix, int s,
-                                     float c, float w, Pt& p) {
+// RK update of one value from loaded operands.
+template <int KIND>
+__device__ __forceinline__ void put(float k, float y, float u, float* out, float* acc, size_t i,
+                                    float c, float w) {
+  if (KIND == kStageFirst) {
+    out[i] = fmaf(c, k, y);
+  } else if (KIND == kStageLast) {
+    out[i] = rk_last(k, y, u, c);
+  } else {
+    out[i] = fmaf(c, k, u);
+    if (KIND == kStageSecond) acc[i] = rk_acc(k, y, u, w);
+  }
+}
+
+constexpr int kBands = 5;  // free surface, left, right, top (CPML), bottom
+
+struct Args {
+  SCoef C;
+  SFields in, out, un, acc;
+  int s;
+  Band edge[kBands];  // 8 rows each
+  Band inner;         // `tr` rows
+  int tr;
+  float c, w;
+};
+
+// One tile. SURF, PML as in rhs(); neither: an interior tile, a thread takes
+// every kRowStep-th row of its column.
+template <int DIR, int KIND, bool SURF, bool PML, bool CPML>
+__device__ __forceinline__ void run_tile(const Args& a, const Tile& tl, float* tile) {
+  const SCoef& C = a.C;
   const int nx = C.nx, nz = C.nz, npd = C.npd, P = C.P;
-  const int it = IN ? 0 : __ldg(C.step);
+  const size_t n = (size_t)nz * P;
+  const int ty = threadIdx.x / kTX, tx = threadIdx.x % kTX, ix = tl.x0 + tx;
+  constexpr int LO = !SURF && DIR == kDirF ? 1 : 3, HI = !SURF && DIR == kDirB ? 1 : 3;
+  stage_tile<5, LO, HI>(tile, a.in.vx, n, tl.x0, tl.z0, PML ? kRowStep : a.tr, nz, P);
+  int iz = tl.z0 + ty;
+  const bool active = ix < tl.x1 && (!PML || ix >= 3) && iz < tl.z1;
+  Pt p;
+  if (active) load_pt<KIND>(p, C, a.un, a.acc, (size_t)iz * P + ix);
+  const bool side = PML && active && min(ix - 3, nx - 4 - ix) < npd;
+  const bool band = PML && active && (iz >= nz - 3 - npd || (CPML && iz <= npd + 2));
+  const size_t si = (size_t)iz * C.Ps + (side ? xstrip_col(ix, nx, npd) : 0);
+  const size_t zi = (size_t)zeta_row<CPML>(iz, nz, npd) * P + ix;
+  float xa[4], ux[4], za[4], uz[4];
+  float4 px = make_float4(0.f, 0.f, 0.f, 0.f), pz = px;
+  if (side) {
+    load_ade<KIND>(xa, ux, a.in.x, a.un.x, a.acc.x, si);
+    px = __ldg(C.pmlx + ix);
+  }
+  if (band) {
+    load_ade<KIND>(za, uz, a.in.z, a.un.z, a.acc.z, zi);
+    pz = __ldg(C.pmlz + iz);
+  }
+  const int2 src = __ldg(C.src_pos);
+  // the source's 5x5 cells touch this tile
+  const bool near_src = src.x >= 0 && src.x >= tl.x0 - 2 && src.x < tl.x0 + kTX + 2 &&
+                        src.y >= tl.z0 - 2 && src.y < tl.z1 + 2;
+  cp_async_wait_all();
+  __syncthreads();
+  if (!active) return;
 #pragma unroll 1
-  for (int k = 0; k < kTZ / kBY; ++k) {
-    const int lz = 3 + threadIdx.y + k * kBY, iz = r0 + lz;
-    if (iz > nz - 4) return;
-    auto A = [&](int q, int dz, int dx) { return tile[q][lz + dz][3 + threadIdx.x + dx]; };
+  for (;;) {
     const size_t i = (size_t)iz * P + ix;
-    if (k > 0) load_pt<KIND>(p, C, un, acc, i);
+    const TileAcc<5> T(tile, 3 + iz - tl.z0, 4 + tx);
+    auto A = [&](int q, int dz, int dx) { return T.at(q, dz, dx); };
     auto K = [&](int cf) { return p.k[cf]; };
-    Out o = rhs<DIR, IN, CPML>(C, in, A, K, iz, ix);
-    if (!IN) {
+    Out o = rhs<DIR, SURF, PML, CPML>(C, A, K, iz, ix, side, band, xa, za, px, pz);
+    if (near_src) {
       // explosive source on both normal stresses (src/pml_fs_kernels.cu:22-26)
-      const int sx = ix - C.srcx, sz = iz - C.srcz;
-      if (C.srcx >= 0 && sx >= -2 && sx <= 2 && sz >= -2 && sz <= 2 && it >= 0 && it < C.src_steps) {
-        const float q = __ldg(C.src_amp + (size_t)it * 4 + s) * kSrcW[(sz + 2) * 5 + (sx + 2)];
+      const int it = (C.step ? __ldg(C.step) : 0) + C.it_off, sx = ix - src.x, sz = iz - src.y;
+      if (sx >= -2 && sx <= 2 && sz >= -2 && sz <= 2 && it >= 0 && it < C.src_steps) {
+        const float q = __ldg(C.src_amp + (size_t)it * 4 + a.s) * c_srcw[(sz + 2) * 5 + (sx + 2)];
         o.sx += q;
         o.sz += q;
       }
     }
-    store5<KIND>(o, p, [&](int q) { return A(q, 0, 0); }, out, acc, i, c, w);
-    if (!IN && min(ix - 3, nx - 4 - ix) < npd) {
-      const size_t si = (size_t)iz * C.Ps + xstrip_col(ix, nx, npd);
-      upd<KIND>(o.XV0, in.x[0], un.x[0], out.x[0], acc.x[0], si, c, w);
-      upd<KIND>(o.XV1, in.x[1], un.x[1], out.x[1], acc.x[1], si, c, w);
-      upd<KIND>(o.XE0, in.x[2], un.x[2], out.x[2], acc.x[2], si, c, w);
-      upd<KIND>(o.XE1, in.x[3], un.x[3], out.x[3], acc.x[3], si, c, w);
-    }
-    if (!IN && (iz >= nz - 3 - npd || (CPML && iz <= npd + 2))) {
-      const size_t zi = (size_t)zeta_row<CPML>(iz, nz, npd) * P + ix;
-      upd<KIND>(o.ZV0, in.z[0], un.z[0], out.z[0], acc.z[0], zi, c, w);
-      upd<KIND>(o.ZV1, in.z[1], un.z[1], out.z[1], acc.z[1], zi, c, w);
-      upd<KIND>(o.ZE0, in.z[2], un.z[2], out.z[2], acc.z[2], zi, c, w);
-      upd<KIND>(o.ZE1, in.z[3], un.z[3], out.z[3], acc.z[3], zi, c, w);
-    }
-  }
-}
-
-template <int DIR, int KIND, bool CPML>
-__global__ void __launch_bounds__(kBX * kBY, 4) k_stage(SCoef C, SFields in, SFields out,
-                                                                      SFields un, SFields acc, int s,
-                                                                      float c, float w) {
-  __shared__ __align__(16) float tile[5][kHH][kHW];
-  const int nx = C.nx, nz = C.nz, npd = C.npd, P = C.P;
-  const int c0 = blockIdx.x * kBX, r0 = blockIdx.y * kTZ;
-  const int ix = 3 + c0 + threadIdx.x, iz0 = r0 + 3 + threadIdx.y;
-  // the first row's point-wise operands, in flight together with the tile
-  Pt p;
-  if (ix <= nx - 4 && iz0 <= nz - 4) load_pt<KIND>(p, C, un, acc, (size_t)iz0 * P + ix);
-  // Stage the tile: rows r0.. (below nz), float4 columns c0.. (below P; the
-  // pitch is a multiple of 32 floats, so every float4 lies in one row and no
-  // column at or beyond nx is ever read back). 250 of the 256 threads each own
-  // one float4 column of every 25th tile row.
-  {
-    constexpr int kV = kHW / 4, kRowsPerPass = (kBX * kBY) / kV;
-    const int tid = threadIdx.y * kBX + threadIdx.x, vr = tid / kV, vc = (tid - vr * kV) * 4;
-    if (vr < kRowsPerPass && c0 + vc < P) {
+    const float k[5] = {o.vx, o.vz, o.sx, o.sz, o.sxz};
 #pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        const float* f = q == kVX ? in.vx : q == kVZ ? in.vz : q == kSX ? in.sx : q == kSZ ? in.sz : in.sxz;
+    for (int q = 0; q < 5; ++q)
+      put<KIND>(k[q], T.at(q, 0, 0), p.u[q], a.out.vx + q * n, a.acc.vx + q * n, i, a.c, a.w);
+    if (PML) {
+      const float kx[4] = {o.XV0, o.XV1, o.XE0, o.XE1}, kz[4] = {o.ZV0, o.ZV1, o.ZE0, o.ZE1};
 #pragma unroll
-        for (int rr = vr; rr < kHH; rr += kRowsPerPass)
-          if (r0 + rr < nz)
-            *reinterpret_cast<float4*>(&tile[q][rr][vc]) =
-                __ldg(reinterpret_cast<const float4*>(f + (size_t)(r0 + rr) * P + c0 + vc));
+      for (int q = 0; q < 4; ++q) {
+        if (side) put<KIND>(kx[q], xa[q], ux[q], a.out.x[q], a.acc.x[q], si, a.c, a.w);
+        if (band) put<KIND>(kz[q], za[q], uz[q], a.out.z[q], a.acc.z[q], zi, a.c, a.w);
       }
     }
-  }
-  __syncthreads();
-  if (ix > nx - 4) return;
-  // Blocks whose cells are all at least three rows below the free surface (with
-  // CPML: below the top band), in no absorbing strip and away from the source
-  // take the branch-free body.
-  const bool interior = r0 >= (CPML ? npd : 3) && r0 + kTZ + 2 < nz - 3 - npd && c0 >= npd &&
-                        c0 + kBX + 2 <= nx - 4 - npd &&
-                        (C.srcx < 0 || C.srcx + 2 < c0 + 3 || C.srcx - 2 > c0 + kBX + 2 ||
-                         C.srcz + 2 < r0 + 3 || C.srcz - 2 > r0 + kTZ + 2);
-  if (interior)
-    rows<DIR, KIND, true, CPML>(C, in, out, un, acc, tile, r0, ix, s, c, w, p);
-  else
-    rows<DIR, KIND, false, CPML>(C, in, out, un, acc, tile, r0, ix, s, c, w, p);
-}
-
-__global__ void k_finish(SCoef C, SFields U) {
-  const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-  const int it = *C.step;
-  if (ix < C.nx) {
-    const float v = U.vz[(size_t)C.rec_row * C.P + ix];
-    if (!isfinite(v)) atomicOr(C.status, 1);
-    if (C.rec != nullptr && C.gap > 0 && it % C.gap == 0) {
-      const int j = it / C.gap;
-      if (j < C.rec_cap) C.rec[(size_t)j * C.nx + ix] = v;
+    if (KIND == kStageLast && iz == C.rec_row) {  // the receiver row (src/main.cu:284-311)
+      const float v = rk_last(k[kVZ], T.at(kVZ, 0, 0), p.u[kVZ], a.c);
+      const int it = (C.step ? __ldg(C.step) : 0) + C.it_off, j = C.gap > 0 ? it / C.gap : 0;
+      if (!isfinite(v)) atomicOr(C.status, 1);
+      if (C.rec != nullptr && C.gap > 0 && j * C.gap == it && j < C.rec_cap)
+        C.rec[(size_t)j * nx + ix] = v;
     }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned prev = atomicAdd(C.done, 1u);
-    if (prev == gridDim.x - 1) {
-      *C.done = 0u;
-      *C.step = it + 1;
-      __threadfence();
-    }
+    if (PML) return;
+    iz += kRowStep;
+    if (iz >= tl.z1) return;
+    load_pt<KIND>(p, C, a.un, a.acc, (size_t)iz * P + ix);
   }
 }
 
-__global__ void k_set_step(int* step, unsigned* done, int it) {
-  *step = it;
-  *done = 0u;
+template <int MINB, int DIR, int KIND, bool CPML>
+__global__ void __launch_bounds__(kThreads, MINB) k_stage(const __grid_constant__ Args a) {
+  extern __shared__ __align__(16) float tile[];
+  const int b = blockIdx.x;
+  if (b >= a.inner.first) {
+    run_tile<DIR, KIND, false, false, CPML>(a, tile_of(a.inner, b, a.tr), tile);
+  } else if (!CPML && b < a.edge[1].first) {
+    run_tile<DIR, KIND, true, true, CPML>(a, tile_of(a.edge[0], b, kRowStep), tile);
+  } else {
+    int k = 1;
+#pragma unroll
+    for (int q = 2; q < kBands; ++q)
+      if (b >= a.edge[q].first) k = q;
+    run_tile<DIR, KIND, false, true, CPML>(a, tile_of(a.edge[k], b, kRowStep), tile);
+  }
 }
 
-template <int DIR, int KIND>
+__global__ void k_set_step(int* step, int it) { *step = it; }
+__global__ void k_advance_step(int* step, int n) { *step += n; }
+
+template <int MINB, int DIR, int KIND>
 cudaError_t launch_t(const SCoef& C, const SFields& in, const SFields& out, const SFields& un,
-                     const SFields& acc, int s, cudaStream_t st) {
-  const dim3 grid(unsigned((C.nx - 6 + kBX - 1) / kBX), unsigned((C.nz - 6 + kTZ - 1) / kTZ));
-  const float c = C.rk_c[s], w = KIND == kStageSecond ? C.rk_w : 0.f;
+                     const SFields& acc, cudaStream_t st) {
+  Args a;
+  a.C = C; a.in = in; a.out = out; a.un = un; a.acc = acc;
+  a.s = KIND;
+  a.c = C.rk_c[KIND];
+  a.w = KIND == kStageSecond ? C.rk_w : 0.f;
+  const int nx = C.nx, nz = C.nz, npd = C.npd;
+  // tall tiles stage fewer halo rows, short ones give a small grid enough blocks
+  // (us a step at 8 / 16 / 24 / 32 rows: 200x200 19.2 / 19.6 / 19.6 / 19.7, 600x600
+  // 37.2 / 35.1 / 37.2 / 37.7, 2048x2048 328 / 314 / 307 / 312)
+  a.tr = MINB == 5 ? 3 * kRowStep : (long long)nx * nz < 100000 ? kRowStep : 2 * kRowStep;
+  // rows 3..nz-4: 8 rows under the free surface, the bottom band (and the top
+  // band with CPML); columns 3..nx-4: the side strips in whole tile columns
+  const int z0 = C.cpml ? 3 : std::min(3 + kRowStep, nz - 3), z1 = nz - 3;
+  int xl = std::min(ceil_div(3 + npd, kTX) * kTX, nx - 3), xr = std::max((nx - 3 - npd) / kTX * kTX, xl);
+  if (xr - xl < 4) xl = xr = nx - 3;  // no interior columns: all in the left band
+  const int zt = C.cpml ? std::min(std::max(npd + 3, z0), z1) : z0;
+  const int zb = std::min(std::max(nz - 3 - npd, zt), z1);
+  int n = make_band(a.edge[0], 0, nx - 3, 3, z0, kRowStep, 0);
+  n = make_band(a.edge[1], 0, xl, z0, z1, kRowStep, n);
+  n = make_band(a.edge[2], xr, nx - 3, z0, z1, kRowStep, n);
+  n = make_band(a.edge[3], xl, xr, z0, zt, kRowStep, n);
+  n = make_band(a.edge[4], xl, xr, zb, z1, kRowStep, n);
+  n = make_band(a.inner, xl, xr, zt, zb, a.tr, n);
   if (C.cpml)
-    k_stage<DIR, KIND, true><<<grid, dim3(kBX, kBY), 0, st>>>(C, in, out, un, acc, s, c, w);
+    k_stage<MINB, DIR, KIND, true><<<unsigned(n), kThreads, tile_smem(a.tr), st>>>(a);
   else
-    k_stage<DIR, KIND, false><<<grid, dim3(kBX, kBY), 0, st>>>(C, in, out, un, acc, s, c, w);
+    k_stage<MINB, DIR, KIND, false><<<unsigned(n), kThreads, tile_smem(a.tr), st>>>(a);
   return cudaGetLastError();
+}
+
+template <int MINB, int DIR>
+cudaError_t launch_d(const SCoef& C, const SFields& in, const SFields& out, const SFields& un,
+                     const SFields& acc, int stage, cudaStream_t st) {
+  switch (stage) {
+    case 0: return launch_t<MINB, DIR, kStageFirst>(C, in, out, un, acc, st);
+    case 1: return launch_t<MINB, DIR, kStageSecond>(C, in, out, un, acc, st);
+    case 2: return launch_t<MINB, DIR, kStageThird>(C, in, out, un, acc, st);
+    default: return launch_t<MINB, DIR, kStageLast>(C, in, out, un, acc, st);
+  }
 }
 
 }  // namespace
 
 cudaError_t launch_stage(const SCoef& C, const SFields& in, const SFields& out, const SFields& un,
                          const SFields& acc, int stage, int dir, cudaStream_t st) {
-  if (dir == kDirF) {
-    if (stage == 0) return launch_t<kDirF, kStageFirst>(C, in, out, un, acc, stage, st);
-    if (stage == 1) return launch_t<kDirF, kStageSecond>(C, in, out, un, acc, stage, st);
-    if (stage == 2) return launch_t<kDirF, kStageThird>(C, in, out, un, acc, stage, st);
-    return launch_t<kDirF, kStageLast>(C, in, out, un, acc, stage, st);
-  }
-  if (stage == 0) return launch_t<kDirB, kStageFirst>(C, in, out, un, acc, stage, st);
-  if (stage == 1) return launch_t<kDirB, kStageSecond>(C, in, out, un, acc, stage, st);
-  if (stage == 2) return launch_t<kDirB, kStageThird>(C, in, out, un, acc, stage, st);
-  return launch_t<kDirB, kStageLast>(C, in, out, un, acc, stage, st);
-}
-
-cudaError_t launch_finish(const SCoef& C, const SFields& U, cudaStream_t st) {
-  k_finish<<<unsigned((C.nx + 255) / 256), 256, 0, st>>>(C, U);
-  return cudaGetLastError();
+  // Small grids are one wave or two, bound by the latency of a block, and take the
+  // larger register budget; large ones are bound by memory and take more blocks
+  // per SM (us a step, 3 / 5 blocks: 400x400 23.0 / 30.0, 600x600 35.1 / 40.8,
+  // 800x800 56.6 / 54.6, 1000x1000 104 / 100, 2048x2048 343 / 307, 4096x4096
+  // 1253 / 1068).
+  if ((long long)C.nx * C.nz < 600000)
+    return dir == kDirF ? launch_d<3, kDirF>(C, in, out, un, acc, stage, st)
+                        : launch_d<3, kDirB>(C, in, out, un, acc, stage, st);
+  return dir == kDirF ? launch_d<5, kDirF>(C, in, out, un, acc, stage, st)
+                      : launch_d<5, kDirB>(C, in, out, un, acc, stage, st);
 }
 
 cudaError_t launch_set_step(const SCoef& C, int it, cudaStream_t st) {
-  k_set_step<<<1, 1, 0, st>>>(C.step, C.done, it);
+  k_set_step<<<1, 1, 0, st>>>(C.step, it);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_advance_step(const SCoef& C, int n, cudaStream_t st) {
+  k_advance_step<<<1, 1, 0, st>>>(C.step, n);
   return cudaGetLastError();
 }
 

@@ -27,15 +27,15 @@ struct SCoef {
   const float4* __restrict__ pmlz;  // per row (bottom band; with cpml also the top band)
   const float* __restrict__ src_amp;  // Ricker value per (step, stage): [steps][4]
   int src_steps;
-  int srcx, srcz;                   // source cell (srcx < 0: none)
+  const int2* __restrict__ src_pos; // source cell (x < 0: none)
   float rk_c[4];                    // dt/2, dt/2, dt and k4's weight (rk_once)
   float rk_w;                       // k2's weight (rk_once)
   int gap, rec_cap;
   float* rec;                       // [rec_cap][nx]: solid vz on row rec_row
   int rec_row;                      // 3 (free surface) or 30 (cpml), src/main.cu:303-311
   int cpml;                         // 1: CFS-PML on all four sides, no free surface
-  int* step;                        // device step counter
-  unsigned* done;                   // block arrival counter of the finish kernel
+  int* step;                        // device step counter: the time index of a launch is
+  int it_off;                       // *step + it_off (step null: it_off)
   int* status;                      // sticky non-finite flag
 };
 
@@ -50,14 +50,15 @@ struct SFields {
 };
 
 // RK stage `stage` (0..3) with operator direction `dir` (0 F, 1 B): reads `in`
-// (and U^n = `un`, the accumulator `acc`), writes `out` and the accumulator.
+// (and U^n = `un`, the accumulator `acc`), writes `out` and the accumulator; the
+// last stage records solid vz on row rec_row when the time index is a multiple
+// of gap and flags non-finite values there.
 cudaError_t launch_stage(const SCoef& C, const SFields& in, const SFields& out, const SFields& un,
                          const SFields& acc, int stage, int dir, cudaStream_t st);
-// Records solid vz on row rec_row when the step index is a multiple of gap, flags
-// non-finite values and advances the device step counter.
-cudaError_t launch_finish(const SCoef& C, const SFields& U, cudaStream_t st);
 // Sets the device step counter.
 cudaError_t launch_set_step(const SCoef& C, int it, cudaStream_t st);
+// Adds n to the device step counter (the end of a captured run of n steps).
+cudaError_t launch_advance_step(const SCoef& C, int n, cudaStream_t st);
 
 }  // namespace solid
 }  // namespace mfdm

@@ -18,9 +18,9 @@
 //   interior tiles of 32 columns x `tr` rows, which take a branch-free body.
 #include <algorithm>
 
-#include "mfdm_async.cuh"
 #include "mfdm_device.cuh"
 #include "mfdm_kernels.h"
+#include "mfdm_tile.cuh"
 
 // This file is compiled four times: with a register budget for 3 (as it is), 2
 // (mfdm_stage_b2.cu) and 5 (mfdm_stage_b4.cu, mfdm_stage_b4o.cu) resident blocks
@@ -36,27 +36,9 @@ namespace mfdm {
 namespace MFDM_STAGE_NS {
 namespace {
 
-constexpr bool kOnce = MFDM_STAGE_ONCE;
-constexpr int kThreads = 256;
-constexpr int kTX = 32;                   // columns of a tile
-constexpr int kW = kTX + 8;               // staged columns x0-4 .. x0+35
-constexpr int kRowStep = kThreads / kTX;  // rows between a thread's cells (8)
-constexpr int kTileRowsMax = 48;          // tallest interior tile
-// Shared memory of an interior tile: tr + 6 rows of 5 fields, the columns and a
-// 4-column halo each side (more than a PML tile or an interface block needs).
-constexpr size_t tile_smem(int tr) { return size_t(tr + 6) * 5 * (kTX + 8) * sizeof(float); }
+using namespace tiles;
 
-// Stage input staged as [row][field][column]: every neighbour of a cell is its
-// base plus a compile-time offset.
-template <int NST>
-struct TileAcc {
-  const float* base;
-  __device__ __forceinline__ TileAcc(const float* tile, int lz, int c)
-      : base(tile + lz * (NST * kW) + c) {}
-  __device__ __forceinline__ float at(int f, int dz, int dx) const {
-    return base[dz * (NST * kW) + f * kW + dx];
-  }
-};
+constexpr bool kOnce = MFDM_STAGE_ONCE;
 struct FluidTile : TileAcc<3> {
   using TileAcc<3>::TileAcc;
   __device__ __forceinline__ float fvx(int dz, int dx) const { return at(0, dz, dx); }
@@ -78,27 +60,6 @@ __device__ __forceinline__ int2 source_of(const Coef& C, int shot) {
 }
 __device__ __forceinline__ float4 pml_at(const float4* t, size_t so, int i) {
   return __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(t) + so) + i);
-}
-
-// Stages rows z0-LO .. z0+tr+HI-1 of the NST fields at `f` (plane stride `plane`,
-// `rows` rows of pitch P), columns x0-4 .. x0+35 (x0 a multiple of 4), with
-// 16-byte asynchronous copies; zero outside the arrays. Every thread owns one
-// float4 column of every kPass-th row.
-template <int NST, int LO, int HI>
-__device__ __forceinline__ void stage_tile(float* tile, const float* f, size_t plane, int x0, int z0,
-                                           int tr, int rows, int P) {
-  constexpr int kV = kW / 4, kPer = NST * kV, kPass = kThreads / kPer;
-  const int rr = threadIdx.x / kPer, e = threadIdx.x - rr * kPer, q = e / kV, vc = (e - q * kV) * 4;
-  const int col = x0 - 4 + vc;
-  const bool in_x = col >= 0 && col < P;
-  const float* src = f + q * plane + col;
-  uint32_t dst = smem_addr(tile + ((3 - LO + rr) * NST + q) * kW + vc);
-  if (rr < kPass)
-    for (int r = z0 - LO + rr; r < z0 + tr + HI; r += kPass, dst += kPass * NST * kW * 4) {
-      const bool ok = in_x && r >= 0 && r < rows;
-      cp_async16(dst, ok ? src + (size_t)r * P : f, ok);
-    }
-  cp_async_commit();
 }
 
 // Point-wise operands of one cell: `u`, U^n (second and third stage) or the
@@ -154,11 +115,6 @@ __device__ __forceinline__ void rk_store(float k, float y, float u, float q, flo
   }
 }
 
-// A rectangle of tiles: columns from x0 (`ntx` tiles a row) to below x1, rows
-// z0..z1-1; its blocks are [first, next rectangle's first).
-struct Band {
-  int first, x0, x1, ntx, z0, z1;
-};
 constexpr int kBands = 6;  // fluid: left, right, top (four-side CPML); solid: left, right, bottom
 
 struct StageArgs {
@@ -173,19 +129,6 @@ struct StageArgs {
   int tr;
   float cc, w;
 };
-
-struct Tile {
-  int x0, x1, z0, z1;
-};
-__device__ __forceinline__ Tile tile_of(const Band& b, int blk, int tr) {
-  const int k = blk - b.first, bz = k / b.ntx;
-  Tile t;
-  t.x0 = b.x0 + (k - bz * b.ntx) * kTX;
-  t.x1 = b.x1;
-  t.z0 = b.z0 + bz * tr;
-  t.z1 = min(t.z0 + tr, b.z1);
-  return t;
-}
 
 // One fluid (solid) tile: rows 6..nz_f-4 (3..nz_s-4; from row 3
 // with four-side CPML), where the plain operators hold. PML: cells may lie in an
@@ -526,15 +469,6 @@ __global__ void __launch_bounds__(kThreads, MFDM_STAGE_BLOCKS)
 int tile_rows_of(const Coef& C) {
   const int tr = (stage_seg_rows(C) + kRowStep - 1) / kRowStep * kRowStep;
   return tr < kTileRowsMax ? tr : kTileRowsMax;
-}
-
-int ceil_div(int a, int b) { return (a + b - 1) / b; }
-
-// Columns [x0, x1) x rows [z0, z1) in tiles of tz rows, blocks from `first` on.
-int make_band(Band& b, int x0, int x1, int z0, int z1, int tz, int first) {
-  const bool empty = x1 <= x0 || z1 <= z0;
-  b = {first, x0, x1, empty ? 1 : ceil_div(x1 - x0, kTX), z0, empty ? z0 : z1};
-  return first + (empty ? 0 : b.ntx * ceil_div(z1 - z0, tz));
 }
 
 template <int DIR, int KIND, bool CPML>
