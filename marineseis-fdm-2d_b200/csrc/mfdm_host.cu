@@ -138,7 +138,7 @@ struct mfdm_model {
   std::vector<ShotCfg> shots;  // per-shot source, frequency and PML beta0
   bool batch = false;          // opened with mfdm_open_batch
   size_t region = 0;           // bytes of one shot's state region
-  int* d_srcpos = nullptr;     // per-shot source cells (batch handles)
+  int* d_srcpos = nullptr;     // per-shot source cells (x < 0: none)
   cudaStream_t stream = nullptr;
   HostModel cfg;  // scalars (arrays released after upload)
   int P = 0, Ps = 0, nz = 0, gap = 1;
@@ -448,6 +448,15 @@ int check_status(mfdm_model* m) {
   return status_error(st, "non-finite values reached the interface rows");
 }
 
+// Writes a plain handle's source cell to the device, where the kernels read it.
+int plain_source(mfdm_model* m) {
+  const HostModel& c = m->cfg;
+  const int pos[2] = {c.srcx.empty() ? -1 : c.srcx[size_t(m->isrc)],
+                      c.srcx.empty() ? 0 : c.srcz[size_t(m->isrc)]};
+  MFDM_CU(cudaMemcpyAsync(m->d_srcpos, pos, sizeof pos, cudaMemcpyHostToDevice, m->stream));
+  return MFDM_OK;
+}
+
 // Uploads the model arrays, the FP64-derived PML tables and normals, and the
 // scalars of `h` into the buffers of `m` (shape already checked).
 int upload_model(mfdm_model* m, const HostModel& h) {
@@ -531,8 +540,7 @@ int upload_model(mfdm_model* m, const HostModel& h) {
   c.vp_max = h.vp_max; c.rc = h.rc; c.beta0 = h.beta0; c.bdy = h.bdy;
   c.srcx = h.srcx; c.srcz = h.srcz;
   if (m->isrc >= int(c.srcx.size())) m->isrc = 0;
-  C.srcx = c.srcx.empty() ? -1 : c.srcx[size_t(m->isrc)];
-  C.srcz = c.srcx.empty() ? 0 : c.srcz[size_t(m->isrc)];
+  if (!m->batch && (rc = plain_source(m)) != MFDM_OK) return rc;
   // The source table depends on fpeak and dt: rebuild it.
   if (m->d_src) cudaFree(m->d_src);
   m->d_src = nullptr;
@@ -650,9 +658,9 @@ int build(mfdm_model* m, HostModel&& h, int device, const std::vector<ShotCfg>* 
   C.shot_stride = roff / sizeof(float);
   C.src_stride = 0;
   C.rec_stride = 0;
-  C.src_pos = nullptr;
+  m->d_srcpos = reinterpret_cast<int*>(F(o_srcpos));
+  C.src_pos = reinterpret_cast<const int2*>(m->d_srcpos);
   if (m->batch) {
-    m->d_srcpos = reinterpret_cast<int*>(F(o_srcpos));
     std::vector<int> pos(size_t(2) * m->nshots);
     for (int b = 0; b < m->nshots; ++b) {
       pos[size_t(2 * b)] = m->shots[size_t(b)].x;
@@ -660,7 +668,6 @@ int build(mfdm_model* m, HostModel&& h, int device, const std::vector<ShotCfg>* 
     }
     MFDM_CU(cudaMemcpyAsync(m->d_srcpos, pos.data(), pos.size() * sizeof(int),
                             cudaMemcpyHostToDevice, m->stream));
-    C.src_pos = reinterpret_cast<const int2*>(m->d_srcpos);
   }
   if ((rc = upload_model(m, h)) != MFDM_OK) return rc;
   MFDM_CU(mfdm::launch_set_step(m->C, 0, m->stream));
@@ -907,10 +914,8 @@ int mfdm_set_shot(mfdm_model* m, int isrc, int reset_state) {
     return fail(MFDM_ERR_ARG, "shot index out of range");
   DeviceGuard g(m->device);
   m->isrc = isrc;
-  m->C.srcx = m->cfg.srcx.empty() ? -1 : m->cfg.srcx[size_t(isrc)];
-  m->C.srcz = m->cfg.srcx.empty() ? 0 : m->cfg.srcz[size_t(isrc)];
-  release_graph(m);  // the source position is baked into the kernel arguments
-  int rc;
+  int rc = plain_source(m);  // read on the device: the captured steps stay
+  if (rc != MFDM_OK) return rc;
   // every state set, the stage buffers and the accumulator (the coefficient block is untouched)
   if (reset_state && (rc = clear_state(m)) != MFDM_OK) return rc;
   return rewind(m);

@@ -80,3 +80,6 @@ def test_a_new_shot_keeps_nothing_of_the_last(mfdm):
 
     solid = make(129, 60, 13, 2)
     shots(lambda: mfdm.SolidSolver.from_model(solid), ["solid_vx", "solid_sz"])
+    both = modelgen.curvilinear(160, 121, nt=NT)
+    both.src_x, both.src_z = [60, 100], [both.src_z[0]] * 2
+    shots(lambda: mfdm.Solver.from_model(both), ["solid_vx", "fluid_p"])
