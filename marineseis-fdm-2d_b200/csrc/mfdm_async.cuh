@@ -22,4 +22,16 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// Programmatic dependent launch. A grid launched with the attribute starts when
+// every block of the grid before it on the stream has called launch_dependents()
+// (or ended); wait_previous() returns when that grid has ended and its memory is
+// visible. What a previous grid of the chain writes is read after it, and not
+// through the read-only cache, which assumes data constant from the launch on.
+__device__ __forceinline__ void launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 }  // namespace mfdm

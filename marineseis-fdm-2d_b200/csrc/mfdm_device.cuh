@@ -68,6 +68,7 @@ struct Coef {
   float* rec;                       // [rec_cap][3][nx]: solid vx, solid vz, fluid p
   int* step;                        // device step counter: the time index of a launch is
   int it_off;                       // *step + it_off (step null: it_off)
+  int chain;                        // may start as the stage launch before it on the stream ends
   int* status;                      // sticky error word (non-finite detector)
   int seg;                          // rows per interior tile of the stage launches (0: by size)
   int variant;                      // stage kernel build: 2, 3 or 4 (0: by size)
@@ -160,25 +161,34 @@ __device__ __forceinline__ float over_rho(float x, float r) {
 #endif
 }
 
-// Direct reads of the stage input (the interface strip and the gradient kernels).
-struct FluidGlobal {
+// Direct reads of the stage input through `Ld` (the stage kernels' row blocks; the
+// gradient kernels, whose input no launch beside them writes, through the
+// read-only cache).
+struct ReadOnly {
+  __device__ __forceinline__ float operator()(const float* p) const { return __ldg(p); }
+};
+template <class Ld>
+struct FluidAt {
   const float *vx, *vz, *p;
   size_t base;
   int P;
-  __device__ __forceinline__ float fvx(int dz, int dx) const { return __ldg(vx + base + (ptrdiff_t)dz * P + dx); }
-  __device__ __forceinline__ float fvz(int dz, int dx) const { return __ldg(vz + base + (ptrdiff_t)dz * P + dx); }
-  __device__ __forceinline__ float fp(int dz, int dx) const { return __ldg(p + base + (ptrdiff_t)dz * P + dx); }
+  __device__ __forceinline__ float fvx(int dz, int dx) const { return Ld()(vx + base + (ptrdiff_t)dz * P + dx); }
+  __device__ __forceinline__ float fvz(int dz, int dx) const { return Ld()(vz + base + (ptrdiff_t)dz * P + dx); }
+  __device__ __forceinline__ float fp(int dz, int dx) const { return Ld()(p + base + (ptrdiff_t)dz * P + dx); }
 };
-struct SolidGlobal {
+template <class Ld>
+struct SolidAt {
   const float *vx, *vz, *sx, *sz, *sxz;
   size_t base;
   int P;
-  __device__ __forceinline__ float svx(int dz, int dx) const { return __ldg(vx + base + (ptrdiff_t)dz * P + dx); }
-  __device__ __forceinline__ float svz(int dz, int dx) const { return __ldg(vz + base + (ptrdiff_t)dz * P + dx); }
-  __device__ __forceinline__ float ssx(int dz, int dx) const { return __ldg(sx + base + (ptrdiff_t)dz * P + dx); }
-  __device__ __forceinline__ float ssz(int dz, int dx) const { return __ldg(sz + base + (ptrdiff_t)dz * P + dx); }
-  __device__ __forceinline__ float ssxz(int dz, int dx) const { return __ldg(sxz + base + (ptrdiff_t)dz * P + dx); }
+  __device__ __forceinline__ float svx(int dz, int dx) const { return Ld()(vx + base + (ptrdiff_t)dz * P + dx); }
+  __device__ __forceinline__ float svz(int dz, int dx) const { return Ld()(vz + base + (ptrdiff_t)dz * P + dx); }
+  __device__ __forceinline__ float ssx(int dz, int dx) const { return Ld()(sx + base + (ptrdiff_t)dz * P + dx); }
+  __device__ __forceinline__ float ssz(int dz, int dx) const { return Ld()(sz + base + (ptrdiff_t)dz * P + dx); }
+  __device__ __forceinline__ float ssxz(int dz, int dx) const { return Ld()(sxz + base + (ptrdiff_t)dz * P + dx); }
 };
+using FluidGlobal = FluidAt<ReadOnly>;
+using SolidGlobal = SolidAt<ReadOnly>;
 
 // Centre-cell coefficients of a fluid / solid cell (metric at the cell's global row).
 struct FluidCoefs { float xix, xiz, zex, zez, rho, K; };

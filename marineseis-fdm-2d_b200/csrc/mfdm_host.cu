@@ -395,8 +395,10 @@ int ensure_capacity(mfdm_model* m, int steps) {
 // Enqueues the launches of one step of time index `it`. With `ev` (6 events) an
 // event is recorded before the first launch, after every stage launch and at
 // the step's end. `captured`: the time index is the device step counter + it.
+// `chain`: a stage launch may start as the one before it ends; `after_step`: and
+// so may the first, a step of this handle being the last work on the stream.
 int enqueue_step(mfdm_model* m, int it, cudaStream_t st, cudaEvent_t* ev = nullptr,
-                 bool captured = false) {
+                 bool captured = false, bool chain = true, bool after_step = false) {
   const int d0 = (it & 1) ? mfdm::kDirB : mfdm::kDirF, d1 = 1 - d0;
   const Fields &U = m->S[0], &A = m->S[1], &B = m->S[2], &Acc = m->S[3];
   Coef C = m->C;
@@ -408,6 +410,7 @@ int enqueue_step(mfdm_model* m, int it, cudaStream_t st, cudaEvent_t* ev = nullp
   const int dir[4] = {d0, d1, d0, d1};
   if (ev) MFDM_CU(cudaEventRecord(ev[0], st));
   for (int s = 0; s < 4; ++s) {
+    C.chain = chain && !ev && (s > 0 || after_step);
     MFDM_CU(mfdm::launch_stage(C, *in[s], *out[s], U, Acc, s, dir[s], st));
     if (ev) MFDM_CU(cudaEventRecord(ev[s + 1], st));
   }
@@ -422,7 +425,7 @@ int capture_graph(mfdm_model* m) {
   cudaGraph_t g = nullptr;
   MFDM_CU(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
   int rc = MFDM_OK;
-  for (int k = 0; k < kGraphSteps && rc == MFDM_OK; ++k) rc = enqueue_step(m, k, m->stream, nullptr, true);
+  for (int k = 0; k < kGraphSteps && rc == MFDM_OK; ++k) rc = enqueue_step(m, k, m->stream, nullptr, true, true, k > 0);
   if (rc == MFDM_OK && mfdm::launch_advance_step(m->C, kGraphSteps, m->stream) != cudaSuccess)
     rc = fail(MFDM_ERR_CUDA, "graph capture: step counter");
   cudaError_t e = cudaStreamEndCapture(m->stream, &g);
@@ -929,7 +932,7 @@ int mfdm_update_rk4(mfdm_model* m, int it, void* stream) {
   if (rc != MFDM_OK) return rc;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : m->stream;
   if (st != m->stream) MFDM_CU(cudaStreamSynchronize(m->stream));
-  rc = enqueue_step(m, it, st);
+  rc = enqueue_step(m, it, st, nullptr, false, false);  // the caller's stream: plain launches
   if (rc != MFDM_OK) return rc;
   m->host_step = it + 1;
   return MFDM_OK;
@@ -1182,7 +1185,8 @@ void group_destroy(mfdm_group* g) {
 }
 
 // Enqueues `k` steps of every model on the model's own stream, forked from and
-// joined back into the group stream (the models run concurrently). `graph`:
+// joined back into the group stream (the models run concurrently, so that chained launches gain nothing: 574 us a step of
+// eight uneven models, 560 without). `graph`:
 // graph-step indices 0..k-1 (captured), else the models' own time indices.
 int group_enqueue(mfdm_group* g, int k, bool graph) {
   MFDM_CU(cudaEventRecord(g->fork, g->stream));
@@ -1190,7 +1194,7 @@ int group_enqueue(mfdm_group* g, int k, bool graph) {
     mfdm_model* m = g->ms[i];
     MFDM_CU(cudaStreamWaitEvent(m->stream, g->fork, 0));
     for (int j = 0; j < k; ++j) {
-      const int rc = enqueue_step(m, graph ? j : m->host_step + j, m->stream, nullptr, graph);
+      const int rc = enqueue_step(m, graph ? j : m->host_step + j, m->stream, nullptr, graph, false);
       if (rc != MFDM_OK) return rc;
     }
     if (graph) MFDM_CU(mfdm::launch_advance_step(m->C, k, m->stream));
@@ -1591,6 +1595,7 @@ int enqueue_slot_step(mfdm_model* m, int it, float* base, size_t j, bool last_of
   C.step = nullptr;
   C.it_off = it;
   for (int s = 0; s < 4; ++s) {
+    C.chain = s > 0;
     MFDM_CU(mfdm::launch_stage(C, Y[s], s < 3 ? Y[s + 1] : next, Y[0], Acc, s, dir[s], st));
   }
   return MFDM_OK;
@@ -2073,8 +2078,10 @@ int solid_enqueue_step(mfdm_solid* m, int it, cudaStream_t st, bool captured = f
   const mfdm::solid::SFields* in[4] = {&U, &A, &B, &A};
   const mfdm::solid::SFields* out[4] = {&A, &B, &A, &U};
   const int dir[4] = {d0, d1, d0, d1};
-  for (int s = 0; s < 4; ++s)
+  for (int s = 0; s < 4; ++s) {
+    C.chain = s > 0 || (captured && it > 0);
     MFDM_CU(mfdm::solid::launch_stage(C, *in[s], *out[s], U, Acc, s, dir[s], st));
+  }
   return MFDM_OK;
 }
 

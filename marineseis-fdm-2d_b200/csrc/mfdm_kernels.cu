@@ -35,9 +35,9 @@ __global__ void advance_step_kernel(int* step, int n) { *step += n; }
 // Up to half a million cells the launch is one wave or two and its time is the
 // latency of a block: the build with the larger register budget (3) is faster;
 // beyond, the throughput of the interior tiles decides and the build with more
-// resident blocks (4) is. Measured, us a step, build 3 / 4: 160x121 23.4 / 27.4;
-// 400x400 30.5 / 40.2; 800x400 35.4 / 43.1; 700x700 44.6 / 46.9; 1200x800 98.5 /
-// 83.6; 1400x1300 172 / 160; 2048x1024 188 / 156; 4096x2048 624 / 498.
+// resident blocks (4) is. Measured before launches were chained (mfdm_stage.cu), us
+// a step, build 3 / 4: 160x121 23.4 / 27.4; 400x400 30.5 / 40.2; 800x400 35.4 /
+// 43.1; 700x700 44.6 / 46.9; 1200x800 98.5 / 83.6; 4096x2048 624 / 498.
 int stage_blocks_per_sm(const Coef& C) {
   if (C.variant == 2 || C.variant == 3 || C.variant == 4) return C.variant;
   return launch_cells(C) < 500000 ? 3 : 4;

@@ -280,6 +280,7 @@ extern "C" int mfdm_step_noalloc(const mfdm_device_model* dm, int it, int nsteps
       const int dir[4] = {d0, d1, d0, d1};
       C.it_off = it + k;
       for (int s = 0; s < 4; ++s) {
+        C.chain = s > 0 || k > k0;
         NA_CU(mfdm::launch_stage(C, S[in_set[s]], S[out_set[s]], S[0], S[3], s, dir[s], st));
       }
     }

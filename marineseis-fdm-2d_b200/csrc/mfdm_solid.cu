@@ -16,8 +16,9 @@
 // Bound: HBM. A step moves 96 floats a cell (inputs 4 x 5, U^n 2 x 5, the
 // accumulator 2 x 5, coefficients 4 x 9, outputs 4 x 5), 250 us of 2048x2048 at
 // the measured copy rate. Measured, us a step, against tiles of 32 x 16 that loaded
-// operand by operand and sampled the receivers in a fifth launch: 400x400 50 -> 23,
-// 1000x1000 122 -> 92, 2048x2048 338 -> 300, 4096x4096 1146 -> 1058.
+// operand by operand and sampled the receivers in a fifth launch: 400x400 50 -> 20,
+// 1000x1000 122 -> 87, 2048x2048 338 -> 292, 4096x4096 1146 -> 1057. A launch may
+// start as the one before it ends (mfdm_stage.cu); without: 23, 92, 300, 1058.
 #include <algorithm>
 
 #include "mfdm_device.cuh"
@@ -216,7 +217,10 @@ __device__ __forceinline__ void load_pt(Pt& p, const SCoef& C, const SFields& un
   const size_t n = (size_t)C.nz * C.P;  // the five fields lie one after another
 #pragma unroll
   for (int q = 0; q < 5; ++q)
-    if (KIND != kStageFirst) p.u[q] = __ldg(pu + q * n + i);
+    if (KIND != kStageFirst) p.u[q] = (pu + q * n)[i];
+}
+// The coefficients, which no launch writes.
+__device__ __forceinline__ void load_coef(Pt& p, const SCoef& C, size_t i) {
   p.k[kCXIX] = __ldg(C.xix + i);
   p.k[kCXIZ] = __ldg(C.xiz + i);
   p.k[kCZEX] = __ldg(C.zex + i);
@@ -235,9 +239,9 @@ __device__ __forceinline__ void load_ade(float* y, float* u, float* const* in, f
                                          float* const* acc, size_t i) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    y[q] = __ldg(in[q] + i);
-    if (KIND == kStageSecond || KIND == kStageThird) u[q] = __ldg(un[q] + i);
-    if (KIND == kStageLast) u[q] = __ldg(acc[q] + i);
+    y[q] = in[q][i];
+    if (KIND == kStageSecond || KIND == kStageThird) u[q] = un[q][i];
+    if (KIND == kStageLast) u[q] = acc[q][i];
   }
 }
 
@@ -276,30 +280,29 @@ __device__ __forceinline__ void run_tile(const Args& a, const Tile& tl, float* t
   const size_t n = (size_t)nz * P;
   const int ty = threadIdx.x / kTX, tx = threadIdx.x % kTX, ix = tl.x0 + tx;
   constexpr int LO = !SURF && DIR == kDirF ? 1 : 3, HI = !SURF && DIR == kDirB ? 1 : 3;
-  stage_tile<5, LO, HI>(tile, a.in.vx, n, tl.x0, tl.z0, PML ? kRowStep : a.tr, nz, P);
   int iz = tl.z0 + ty;
   const bool active = ix < tl.x1 && (!PML || ix >= 3) && iz < tl.z1;
   Pt p;
-  if (active) load_pt<KIND>(p, C, a.un, a.acc, (size_t)iz * P + ix);
+  if (active) load_coef(p, C, (size_t)iz * P + ix);
   const bool side = PML && active && min(ix - 3, nx - 4 - ix) < npd;
   const bool band = PML && active && (iz >= nz - 3 - npd || (CPML && iz <= npd + 2));
   const size_t si = (size_t)iz * C.Ps + (side ? xstrip_col(ix, nx, npd) : 0);
   const size_t zi = (size_t)zeta_row<CPML>(iz, nz, npd) * P + ix;
   float xa[4], ux[4], za[4], uz[4];
   float4 px = make_float4(0.f, 0.f, 0.f, 0.f), pz = px;
-  if (side) {
-    load_ade<KIND>(xa, ux, a.in.x, a.un.x, a.acc.x, si);
-    px = __ldg(C.pmlx + ix);
-  }
-  if (band) {
-    load_ade<KIND>(za, uz, a.in.z, a.un.z, a.acc.z, zi);
-    pz = __ldg(C.pmlz + iz);
-  }
   const int2 src = __ldg(C.src_pos);
   // the source's 5x5 cells touch this tile
   const bool near_src = src.x >= 0 && src.x >= tl.x0 - 2 && src.x < tl.x0 + kTX + 2 &&
                         src.y >= tl.z0 - 2 && src.y < tl.z1 + 2;
+  if (side) px = __ldg(C.pmlx + ix);
+  if (band) pz = __ldg(C.pmlz + iz);
+  wait_previous();
+  stage_tile<5, LO, HI>(tile, a.in.vx, n, tl.x0, tl.z0, PML ? kRowStep : a.tr, nz, P);
+  if (active) load_pt<KIND>(p, C, a.un, a.acc, (size_t)iz * P + ix);
+  if (side) load_ade<KIND>(xa, ux, a.in.x, a.un.x, a.acc.x, si);
+  if (band) load_ade<KIND>(za, uz, a.in.z, a.un.z, a.acc.z, zi);
   cp_async_wait_all();
+  launch_dependents();
   __syncthreads();
   if (!active) return;
 #pragma unroll 1
@@ -340,6 +343,7 @@ __device__ __forceinline__ void run_tile(const Args& a, const Tile& tl, float* t
     if (PML) return;
     iz += kRowStep;
     if (iz >= tl.z1) return;
+    load_coef(p, C, (size_t)iz * P + ix);
     load_pt<KIND>(p, C, a.un, a.acc, (size_t)iz * P + ix);
   }
 }
@@ -390,11 +394,8 @@ cudaError_t launch_t(const SCoef& C, const SFields& in, const SFields& out, cons
   n = make_band(a.edge[3], xl, xr, z0, zt, kRowStep, n);
   n = make_band(a.edge[4], xl, xr, zb, z1, kRowStep, n);
   n = make_band(a.inner, xl, xr, zt, zb, a.tr, n);
-  if (C.cpml)
-    k_stage<MINB, DIR, KIND, true><<<unsigned(n), kThreads, tile_smem(a.tr), st>>>(a);
-  else
-    k_stage<MINB, DIR, KIND, false><<<unsigned(n), kThreads, tile_smem(a.tr), st>>>(a);
-  return cudaGetLastError();
+  return C.cpml ? launch_tiles(k_stage<MINB, DIR, KIND, true>, a, n, tile_smem(a.tr), C.chain != 0, st)
+                : launch_tiles(k_stage<MINB, DIR, KIND, false>, a, n, tile_smem(a.tr), C.chain != 0, st);
 }
 
 template <int MINB, int DIR>

@@ -36,6 +36,7 @@ struct SCoef {
   int cpml;                         // 1: CFS-PML on all four sides, no free surface
   int* step;                        // device step counter: the time index of a launch is
   int it_off;                       // *step + it_off (step null: it_off)
+  int chain;                        // may start as the stage launch before it on the stream ends
   int* status;                      // sticky non-finite flag
 };
 

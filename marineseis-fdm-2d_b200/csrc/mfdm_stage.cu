@@ -39,6 +39,14 @@ namespace {
 using namespace tiles;
 
 constexpr bool kOnce = MFDM_STAGE_ONCE;
+// Launches of the other builds may start as the stage launch before them ends: the
+// gap between dependent launches is a fifth of a small grid's stage (us a step,
+// plain / chained: 160x121 24.6 / 21.1, 400x400 30.1 / 28.0, 800x400 36.0 / 31.8,
+// 1200x800 83.8 / 79.7, 2048x1024 177 / 172). A block lets the next grid start once
+// its own operands have arrived, not at its start: the waiting blocks of two later
+// grids would take the slots (160x121 26.4, 800x400 at 16 rows 32.0). Large grids gain nothing
+// (4096x2048 499 / 505).
+constexpr bool kChain = !kOnce;
 struct FluidTile : TileAcc<3> {
   using TileAcc<3>::TileAcc;
   __device__ __forceinline__ float fvx(int dz, int dx) const { return at(0, dz, dx); }
@@ -62,6 +70,13 @@ __device__ __forceinline__ float4 pml_at(const float4* t, size_t so, int i) {
   return __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(t) + so) + i);
 }
 
+// A value that the launch before may have written: not through the read-only
+// cache where this launch may have started before that one's end.
+__device__ __forceinline__ float ld(const float* p) { return kChain ? *p : __ldg(p); }
+struct Ld {
+  __device__ __forceinline__ float operator()(const float* p) const { return ld(p); }
+};
+
 // Point-wise operands of one cell: `u`, U^n (second and third stage) or the
 // accumulator (last stage); `q`, the accumulator where these stages add to it;
 // and the coefficient block's values.
@@ -71,16 +86,21 @@ struct Pt { float u[NST], q[NST], k[NCOEF]; };
 template <int KIND>
 constexpr bool kAdds = !kOnce && (KIND == kStageSecond || KIND == kStageThird);
 
-template <int NST, int NCOEF, int KIND>
+// The coefficients, which no launch writes, and the rest, which the launch before
+// may have written.
+template <int NST, int NCOEF>
+__device__ __forceinline__ void load_coef(Pt<NST, NCOEF>& p, const float* coef, size_t plane, size_t i) {
+#pragma unroll
+  for (int q = 0; q < NCOEF; ++q) p.k[q] = __ldg(coef + q * plane + i);
+}
+template <int KIND, int NST, int NCOEF>
 __device__ __forceinline__ void load_pt(Pt<NST, NCOEF>& p, const float* u, const float* acc,
-                                        size_t plane, size_t i, const float* coef, size_t ci) {
+                                        size_t plane, size_t i) {
 #pragma unroll
   for (int f = 0; f < NST; ++f) {
-    if (KIND != kStageFirst) p.u[f] = __ldg(u + f * plane + i);
+    if (KIND != kStageFirst) p.u[f] = ld(u + f * plane + i);
     if (kAdds<KIND>) p.q[f] = (acc + f * plane)[i];
   }
-#pragma unroll
-  for (int q = 0; q < NCOEF; ++q) p.k[q] = __ldg(coef + q * plane + ci);
 }
 
 // The four ADE values of a strip cell: the stage input's (`y`) and the operands
@@ -90,8 +110,8 @@ __device__ __forceinline__ void load_ade(float* y, float* u, float* qa, float* c
                                          float* const* acc, size_t i) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    y[q] = __ldg(in[q] + i);
-    if (KIND == kStageSecond || KIND == kStageThird) u[q] = __ldg(un[q] + i);
+    y[q] = ld(in[q] + i);
+    if (KIND == kStageSecond || KIND == kStageThird) u[q] = ld(un[q] + i);
     if (KIND == kStageLast) u[q] = acc[q][i];
     if (kAdds<KIND>) qa[q] = acc[q][i];
   }
@@ -142,13 +162,14 @@ __device__ __forceinline__ void fluid_tile(const StageArgs& a, int shot, const T
   const int ty = threadIdx.x / kTX, tx = threadIdx.x % kTX, ix = tl.x0 + tx;
   const float* u = (KIND == kStageLast ? a.acc.fvx : a.un.fvx) + so;
   const float* coef = C.rhof - 4 * nf;  // the fluid coefficient block [6][nz_f][P]
+  if (kChain) wait_previous();
   stage_tile<3, DIR == kDirF ? 1 : 3, DIR == kDirF ? 3 : 1>(
       tile, a.in.fvx + so, nf, tl.x0, tl.z0, PML ? kRowStep : a.tr, nzf, P);
   int iz = tl.z0 + ty;
   const bool active = ix < tl.x1 && (!PML || ix >= 3) && iz < tl.z1;
   Pt<3, 6> p;
-  if (active)
-    load_pt<3, 6, KIND>(p, u, a.acc.fvx + so, nf, (size_t)iz * P + ix, coef, (size_t)iz * P + ix);
+  if (active) load_pt<KIND>(p, u, a.acc.fvx + so, nf, (size_t)iz * P + ix);
+  if (active) load_coef(p, coef, nf, (size_t)iz * P + ix);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const bool side = PML && active && min(ix - 3, nx - 4 - ix) < npd;
   const bool top = PML && CPML && active && iz <= npd + 2;  // four-side CPML: rows 3..npd+2
@@ -156,18 +177,15 @@ __device__ __forceinline__ void fluid_tile(const StageArgs& a, int shot, const T
   const size_t zi = so + (size_t)(iz - 3) * P + ix;
   float ade[4], ua[4], qa[4], zade[4], uz[4], qz[4];
   float4 px = zero, pmz = zero;
-  if (side) {
-    load_ade<KIND>(ade, ua, qa, a.in.fx, a.un.fx, a.acc.fx, si);
-    px = pml_at(C.pmlx, so, ix);
-  }
-  if (top) {
-    load_ade<KIND>(zade, uz, qz, a.in.fz, a.un.fz, a.acc.fz, zi);
-    pmz = pml_at(C.pmlzf, so, iz);
-  }
   const int2 src = source_of(C, shot);
   // the source's 5x5 cells touch this tile
   const bool near_src = src.x >= tl.x0 - 2 && src.x < tl.x0 + kTX + 2 && src.y >= tl.z0 - 2 && src.y < tl.z1 + 2;
+  if (side) px = pml_at(C.pmlx, so, ix);
+  if (top) pmz = pml_at(C.pmlzf, so, iz);
+  if (side) load_ade<KIND>(ade, ua, qa, a.in.fx, a.un.fx, a.acc.fx, si);
+  if (top) load_ade<KIND>(zade, uz, qz, a.in.fz, a.un.fz, a.acc.fz, zi);
   cp_async_wait_all();
+  if (kChain) launch_dependents();
   __syncthreads();
   if (!active) return;
 #pragma unroll 1
@@ -195,7 +213,8 @@ __device__ __forceinline__ void fluid_tile(const StageArgs& a, int shot, const T
     }
     iz += kRowStep;
     if (iz >= tl.z1) return;
-    load_pt<3, 6, KIND>(p, u, a.acc.fvx + so, nf, (size_t)iz * P + ix, coef, (size_t)iz * P + ix);
+    load_pt<KIND>(p, u, a.acc.fvx + so, nf, (size_t)iz * P + ix);
+    load_coef(p, coef, nf, (size_t)iz * P + ix);
   }
 }
 
@@ -207,13 +226,14 @@ __device__ __forceinline__ void solid_tile(const StageArgs& a, int shot, const T
   const int ty = threadIdx.x / kTX, tx = threadIdx.x % kTX, ix = tl.x0 + tx;
   const float* u = (KIND == kStageLast ? a.acc.svx : a.un.svx) + so;
   const float* coef = C.rhos - 4 * ns;  // the solid coefficient block [9][nz_s][P]
+  if (kChain) wait_previous();
   stage_tile<5, DIR == kDirF ? 1 : 3, DIR == kDirF ? 3 : 1>(
       tile, a.in.svx + so, ns, tl.x0, tl.z0, PML ? kRowStep : a.tr, nzs, P);
   int iz = tl.z0 + ty;
   const bool active = ix < tl.x1 && (!PML || ix >= 3) && iz < tl.z1;
   Pt<5, 9> p;
-  if (active)
-    load_pt<5, 9, KIND>(p, u, a.acc.svx + so, ns, (size_t)iz * P + ix, coef, (size_t)iz * P + ix);
+  if (active) load_pt<KIND>(p, u, a.acc.svx + so, ns, (size_t)iz * P + ix);
+  if (active) load_coef(p, coef, ns, (size_t)iz * P + ix);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const bool side = PML && active && min(ix - 3, nx - 4 - ix) < npd;
   const bool bottom = PML && active && iz >= zb0;
@@ -221,15 +241,12 @@ __device__ __forceinline__ void solid_tile(const StageArgs& a, int shot, const T
   const size_t szi = so + (size_t)(iz - zb0) * P + ix;
   float xade[4], ux[4], qx[4], zade[4], uz[4], qz[4];
   float4 px = zero, pz = zero;
-  if (side) {
-    load_ade<KIND>(xade, ux, qx, a.in.sx, a.un.sx, a.acc.sx, sxi);
-    px = pml_at(C.pmlx, so, ix);
-  }
-  if (bottom) {
-    load_ade<KIND>(zade, uz, qz, a.in.sz, a.un.sz, a.acc.sz, szi);
-    pz = pml_at(C.pmlz, so, iz);
-  }
+  if (side) px = pml_at(C.pmlx, so, ix);
+  if (bottom) pz = pml_at(C.pmlz, so, iz);
+  if (side) load_ade<KIND>(xade, ux, qx, a.in.sx, a.un.sx, a.acc.sx, sxi);
+  if (bottom) load_ade<KIND>(zade, uz, qz, a.in.sz, a.un.sz, a.acc.sz, szi);
   cp_async_wait_all();
+  if (kChain) launch_dependents();
   __syncthreads();
   if (!active) return;
 #pragma unroll 1
@@ -254,7 +271,8 @@ __device__ __forceinline__ void solid_tile(const StageArgs& a, int shot, const T
     }
     iz += kRowStep;
     if (iz >= tl.z1) return;
-    load_pt<5, 9, KIND>(p, u, a.acc.svx + so, ns, (size_t)iz * P + ix, coef, (size_t)iz * P + ix);
+    load_pt<KIND>(p, u, a.acc.svx + so, ns, (size_t)iz * P + ix);
+    load_coef(p, coef, ns, (size_t)iz * P + ix);
   }
 }
 
@@ -300,16 +318,17 @@ __device__ __forceinline__ void row_block(const StageArgs& a, int shot, int blk,
   float y[5], u[5], q[5], kv[5], xa[4], ux[4], qx[4], za[4], uz[4], qz[4], kx[4], kz[4];
   bool has_E = true;
   size_t xi = 0, zi = 0;
+  if (kChain) wait_previous();
   if (valid) {
     const float4 px = side ? pml_at(C.pmlx, so, ix) : zero;
     if (!solid) {
-      const FluidGlobal A{a.in.fvx + so, a.in.fvz + so, a.in.fp + so, fi, P};
+      const FluidAt<Ld> A{a.in.fvx + so, a.in.fvz + so, a.in.fp + so, fi, P};
       xi = so + (size_t)iz * C.Ps + scol;
       zi = so + (size_t)(iz - 3) * P + ix;
       const float* ub = (KIND == kStageLast ? a.acc.fvx : a.un.fvx) + so;
 #pragma unroll
       for (int f = 0; f < 3; ++f) {
-        y[f] = __ldg(a.in.fvx + so + f * nf + fi);
+        y[f] = ld(a.in.fvx + so + f * nf + fi);
         u[f] = KIND == kStageFirst ? 0.f : ub[f * nf + fi];
         if (kAdds<KIND>) q[f] = (a.acc.fvx + so)[f * nf + fi];
       }
@@ -325,13 +344,13 @@ __device__ __forceinline__ void row_block(const StageArgs& a, int shot, int blk,
       kx[0] = k.V0; kx[1] = k.V1; kx[2] = k.E0; kx[3] = k.E1;
       kz[0] = k.ZV0; kz[1] = k.ZV1; kz[2] = k.ZE0; kz[3] = k.ZE1;
     } else {
-      const SolidGlobal A{a.in.svx + so, a.in.svz + so, a.in.ssx + so, a.in.ssz + so, a.in.ssxz + so, si, P};
+      const SolidAt<Ld> A{a.in.svx + so, a.in.svz + so, a.in.ssx + so, a.in.ssz + so, a.in.ssxz + so, si, P};
       xi = so + (size_t)iz * C.Ps + scol;
       zi = so + (size_t)(iz - zb0) * P + ix;
       const float* ub = (KIND == kStageLast ? a.acc.svx : a.un.svx) + so;
 #pragma unroll
       for (int f = 0; f < 5; ++f) {
-        y[f] = __ldg(a.in.svx + so + f * ns + si);
+        y[f] = ld(a.in.svx + so + f * ns + si);
         u[f] = KIND == kStageFirst ? 0.f : ub[f * ns + si];
         if (kAdds<KIND>) q[f] = (a.acc.svx + so)[f * ns + si];
       }
@@ -361,6 +380,7 @@ __device__ __forceinline__ void row_block(const StageArgs& a, int shot, int blk,
       for (int q = 0; q < 4; ++q) rk_store<KIND>(kz[q], za[q], uz[q], qz[q], oz[q], az[q], zi, a.cc, a.w);
     }
   }
+  if (kChain) launch_dependents();
   float2 n = make_float2(0.f, 0.f);
   if (iface) {  // the whole block is one or is not
     if (valid) {
@@ -510,8 +530,8 @@ cudaError_t launch_one(const Coef& C, const Fields& in, const Fields& out, const
     if (KIND == kStageSecond) a.w = once.w;
     if (KIND == kStageLast) a.cc = once.c;
   }
-  stage_kernel<DIR, KIND, CPML><<<unsigned(n) * unsigned(a.nshots), kThreads, tile_smem(a.tr), st>>>(a);
-  return cudaGetLastError();
+  return launch_tiles(stage_kernel<DIR, KIND, CPML>, a, n * a.nshots, tile_smem(a.tr),
+                      kChain && C.chain != 0, st);
 }
 
 template <int DIR, bool CPML>

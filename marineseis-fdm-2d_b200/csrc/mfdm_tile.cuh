@@ -66,6 +66,24 @@ __device__ __forceinline__ Tile tile_of(const Band& b, int blk, int tr) {
   return t;
 }
 
+// Launches a stage kernel; chained: it may start while the stage launch before it
+// on the stream ends (mfdm_async.cuh).
+template <class Args>
+cudaError_t launch_tiles(void (*kernel)(Args), const Args& a, int blocks, size_t smem, bool chained,
+                         cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(blocks));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Columns [x0, x1) x rows [z0, z1) in tiles of tz rows, blocks from `first` on.

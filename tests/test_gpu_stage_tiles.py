@@ -83,3 +83,21 @@ def test_batch_of_many_cells_matches_one_shot(mfdm):
             ref = s.records()
             for q in rec:
                 assert rel_l2(rec[q], ref[q]) <= TOL, q
+
+
+@pytest.mark.parametrize("nx,nz_f,nz_s,bdy", [(46, 24, 24, 2), (160, 60, 61, 2), (403, 150, 151, 1),
+                                              (1000, 300, 301, 2)])
+def test_chained_launches_equal_plain_ones(mfdm, nx, nz_f, nz_s, bdy):
+    """Captured steps let a stage launch start as the one before it ends; timing
+    each kernel launches them one after the other. The same kernels on the same
+    data: equal bit for bit (both builds below 2.5 M cells, 96 steps)."""
+    m = modelgen.make_model(nx, nz_f, nz_s, npd=20, fpeak=20.0, nt=96, src_x=[nx // 2],
+                            src_z=[nz_f - 8 if nz_f < 40 else nz_f // 2], boundary_type=bdy)
+    out = []
+    for per_kernel in (False, True):
+        with mfdm.Solver.from_model(m) as s:
+            s.set_shot(0)
+            s.time_steps(96, per_kernel=per_kernel)
+            out.append([s.field(n) for n in mfdm.FIELDS] + list(s.records().values()))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
