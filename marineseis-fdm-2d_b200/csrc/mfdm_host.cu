@@ -932,7 +932,7 @@ int mfdm_update_rk4(mfdm_model* m, int it, void* stream) {
   if (rc != MFDM_OK) return rc;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : m->stream;
   if (st != m->stream) MFDM_CU(cudaStreamSynchronize(m->stream));
-  rc = enqueue_step(m, it, st, nullptr, false, false);  // the caller's stream: plain launches
+  rc = enqueue_step(m, it, st, nullptr, false, st == m->stream);  // the caller's stream: plain launches
   if (rc != MFDM_OK) return rc;
   m->host_step = it + 1;
   return MFDM_OK;
