@@ -396,7 +396,8 @@ int ensure_capacity(mfdm_model* m, int steps) {
 // event is recorded before the first launch, after every stage launch and at
 // the step's end. `captured`: the time index is the device step counter + it.
 // `chain`: a stage launch may start as the one before it ends; `after_step`: and
-// so may the first, a step of this handle being the last work on the stream.
+// so may the first as the kernel before it on the stream ends, whichever that is
+// (one that releases nothing early does so by ending).
 int enqueue_step(mfdm_model* m, int it, cudaStream_t st, cudaEvent_t* ev = nullptr,
                  bool captured = false, bool chain = true, bool after_step = false) {
   const int d0 = (it & 1) ? mfdm::kDirB : mfdm::kDirF, d1 = 1 - d0;
@@ -854,7 +855,7 @@ int enqueue_steps(mfdm_model* m, int nsteps) {
       m->dev_step = m->host_step;
       nsteps -= kGraphSteps;
     } else {
-      if ((rc = enqueue_step(m, m->host_step, m->stream)) != MFDM_OK) return rc;
+      if ((rc = enqueue_step(m, m->host_step, m->stream, nullptr, false, true, true)) != MFDM_OK) return rc;
       ++m->host_step;
       --nsteps;
     }
@@ -932,7 +933,7 @@ int mfdm_update_rk4(mfdm_model* m, int it, void* stream) {
   if (rc != MFDM_OK) return rc;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : m->stream;
   if (st != m->stream) MFDM_CU(cudaStreamSynchronize(m->stream));
-  rc = enqueue_step(m, it, st, nullptr, false, st == m->stream);  // the caller's stream: plain launches
+  rc = enqueue_step(m, it, st, nullptr, false, st == m->stream, st == m->stream);  // the caller's stream: plain launches
   if (rc != MFDM_OK) return rc;
   m->host_step = it + 1;
   return MFDM_OK;
