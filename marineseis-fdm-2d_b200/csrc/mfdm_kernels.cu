@@ -60,9 +60,9 @@ cudaError_t launch_stage(const Coef& C, const Fields& in, const Fields& out, con
     case 3: return b3::launch_stage(C, in, out, un, acc, stage, dir, st);
     // Accumulating once a step saves 17 % of the traffic. Below 2.5 million cells
     // the launch is bound by latency and the L2 cache and gains less (us a step,
-    // in every stage / once: 400x400 29.9 / 28.5, 1200x800 83 / 77), and the
+    // in every stage / once: 1200x800 80.2 / 77.1, 1600x1500 192 / 169), and the
     // reference's order of roundings stays; above, DRAM traffic decides
-    // (4096x2048: 568 / 498; 64 shots of 1200x800: 4300 / 3700).
+    // (4096x2048: 570 / 495; 64 shots of 1200x800: 4440 / 3716).
     default:
       return launch_cells(C) < 2500000 ? b4::launch_stage(C, in, out, un, acc, stage, dir, st)
                                        : b4o::launch_stage(C, in, out, un, acc, stage, dir, st);
