@@ -157,7 +157,9 @@ int mfdm_set_field(mfdm_model* m, int field, const float* host);
  * (src/main.cu:94-136) without clearing the wavefield between them and with
  * one frequency for all; here every shot starts from rest and carries its own
  * source cell and Ricker frequency, with the CFS-PML alpha0 = 2 pi fpeak and
- * beta0 that go with it (elements.cu:121-124, 824-873). */
+ * beta0 that go with it (elements.cu:121-124, 824-873). With the same stage
+ * build (the default is one for both) a shot's results are bit for bit those of
+ * the same shot run alone, however many shots step with it. */
 typedef struct mfdm_shot {
   int src_x, src_z;  /* source column and fluid row (src_x < 0: no source) */
   float fpeak;       /* Ricker peak frequency, Hz                           */
@@ -193,8 +195,9 @@ int mfdm_set_tile(mfdm_model* m, int seg_rows);
 /* Selects the stage kernel build by its register budget: 2 or 3 resident blocks
  * per SM (128 or 80 registers: the strip and interface paths spill little, so
  * a small grid's few blocks finish sooner), 4: five blocks per SM (48
- * registers: more loads in flight, faster on large grids); 0 (default): 3 below
- * 0.5 M cells per launch, 4 from there. Results agree to FP32 rounding. */
+ * registers: more loads in flight, faster on large grids); 0 (default): 3 for a
+ * grid below 0.5 M cells, 4 from there, whatever the number of shots. Results
+ * agree to FP32 rounding. */
 int mfdm_set_blocks_per_sm(mfdm_model* m, int blocks);
 
 /* Times every candidate tile height with every build on this handle's model and

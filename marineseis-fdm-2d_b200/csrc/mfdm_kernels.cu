@@ -32,15 +32,22 @@ __global__ void advance_step_kernel(int* step, int n) { *step += n; }
 
 }  // namespace
 
+// The builds contract the strips' and rows' arithmetic differently and their two
+// accumulation forms round differently, so the choice among them follows the grid
+// of one shot alone: a shot's bits do not depend on how many shots step with it,
+// and a batch gives what its shots give alone. (Tile heights change no bits and
+// follow the whole launch.)
 // Up to half a million cells the launch is one wave or two and its time is the
 // latency of a block: the build with the larger register budget (3) is faster;
 // beyond, the throughput of the interior tiles decides and the build with more
 // resident blocks (4) is. Measured before launches were chained (mfdm_stage.cu), us
 // a step, build 3 / 4: 160x121 23.4 / 27.4; 400x400 30.5 / 40.2; 800x400 35.4 /
-// 43.1; 700x700 44.6 / 46.9; 1200x800 98.5 / 83.6; 4096x2048 624 / 498.
+// 43.1; 700x700 44.6 / 46.9; 1200x800 98.5 / 83.6; 4096x2048 624 / 498. Batches by
+// this rule / by the whole launch: 64 of 160x121 171 / 187, 8 of 400x400 141 / 135,
+// 4 of 800x600 180 / 168.
 int stage_blocks_per_sm(const Coef& C) {
   if (C.variant == 2 || C.variant == 3 || C.variant == 4) return C.variant;
-  return launch_cells(C) < 500000 ? 3 : 4;
+  return shot_cells(C) < 500000 ? 3 : 4;
 }
 
 // Short tiles give a small grid enough blocks, tall ones stage fewer halo rows.
@@ -59,12 +66,13 @@ cudaError_t launch_stage(const Coef& C, const Fields& in, const Fields& out, con
     case 2: return b2::launch_stage(C, in, out, un, acc, stage, dir, st);
     case 3: return b3::launch_stage(C, in, out, un, acc, stage, dir, st);
     // Accumulating once a step saves 17 % of the traffic. Below 2.5 million cells
-    // the launch is bound by latency and the L2 cache and gains less (us a step,
+    // a shot is bound by latency and the L2 cache and gains less (us a step,
     // in every stage / once: 1200x800 80.2 / 77.1, 1600x1500 192 / 169), and the
     // reference's order of roundings stays; above, DRAM traffic decides
-    // (4096x2048: 570 / 495; 64 shots of 1200x800: 4440 / 3716).
+    // (4096x2048: 570 / 495). A batch of smaller grids keeps the order of its
+    // shots alone and pays for it (64 shots of 1200x800: 4394 / 3721).
     default:
-      return launch_cells(C) < 2500000 ? b4::launch_stage(C, in, out, un, acc, stage, dir, st)
+      return shot_cells(C) < 2500000 ? b4::launch_stage(C, in, out, un, acc, stage, dir, st)
                                        : b4o::launch_stage(C, in, out, un, acc, stage, dir, st);
   }
 }

@@ -18,11 +18,12 @@ cudaError_t launch_reciprocal(float* a, int rows, int nx, int P, cudaStream_t st
 cudaError_t launch_set_step(const Coef& C, int it, cudaStream_t st);
 // Adds n to the device step counter (the end of a captured run of n steps).
 cudaError_t launch_advance_step(const Coef& C, int n, cudaStream_t st);
-// Cells one stage launch updates, every shot counted.
+// Cells of one shot, and those one stage launch updates, every shot counted.
+inline long long shot_cells(const Coef& C) { return (long long)C.nx * (C.nzf + C.nzs); }
 inline long long launch_cells(const Coef& C) {
-  return (long long)C.nx * (C.nzf + C.nzs) * (C.nshots > 0 ? C.nshots : 1);
+  return shot_cells(C) * (C.nshots > 0 ? C.nshots : 1);
 }
-// The stage build a launch uses: C.variant, or by size when 0 (see mfdm_stage.cu).
+// The stage build a launch uses: C.variant, or by one shot's size when 0.
 int stage_blocks_per_sm(const Coef& C);
 // Rows per interior tile of a stage launch: C.seg, or by size when 0.
 int stage_seg_rows(const Coef& C);
