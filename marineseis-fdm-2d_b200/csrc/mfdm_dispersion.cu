@@ -35,6 +35,7 @@ constexpr int kDR = 64, kDK = 32;    // traces x frequencies of a spectrum block
 constexpr int kDT = 32;              // sample pairs staged at a time
 constexpr int kDGroup = (kDR / 4) * (kDK / 4);
 constexpr int kDThreads = 2 * kDGroup;  // one group takes the odd samples, one the even
+constexpr size_t kDSumSmem = size_t(2) * kDT * kDR * sizeof(double);
 static_assert(kDGroup == 128 && kDT % 2 == 0, "spectrum block");
 
 // The nt roots exp(-2 pi i m / nt).
@@ -317,11 +318,13 @@ extern "C" int mfdm_dispersion_image(const float* gather, int nt, int ntr, const
       (e = cudaMemcpy(dx, offsets, xb, cudaMemcpyHostToDevice)) != cudaSuccess)
     return err(MFDM_ERR_CUDA, cudaGetErrorString(e));
   const bool in_smem = nt <= kMaxTableSmem;
-  const size_t smem = (in_smem ? rb : 0) + size_t(2) * kDT * kDR * sizeof(double);
+  const size_t smem = (in_smem ? rb : 0) + kDSumSmem;
   const dim3 grid(unsigned((ntr + kDR - 1) / kDR), unsigned(ktiles));
   if (in_smem) {
+    // the limit is the kernel's, not the call's: every call sets it to the most any
+    // call needs, so that none lowers it between another thread's setting and launch
     if ((e = cudaFuncSetAttribute(spectrum_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(smem))) != cudaSuccess)
+                                  int(kMaxTableSmem * sizeof(double2) + kDSumSmem))) != cudaSuccess)
       return err(MFDM_ERR_CUDA, cudaGetErrorString(e));
     spectrum_kernel<true><<<grid, kDThreads, smem>>>(dg, nt, ntr, nk, dr, dP);
   } else {
