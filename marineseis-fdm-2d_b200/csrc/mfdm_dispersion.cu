@@ -20,6 +20,7 @@
 // nt 2000, 400 traces, 301 velocities: spectrum 241 us (987 us with a thread per
 // trace and frequency and every term), image 197 us (428 us with a sincos per
 // term), the call 3.8 -> 0.86 ms with the pool below.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -230,13 +231,40 @@ int err(int code, const char* msg) { return mfdm::set_error(code, msg); }
 // against 0.45 ms of kernels. Pools are safe to use from several threads.
 constexpr unsigned long long kPoolKeep = 64ull << 20;
 constexpr int kMaxDevices = 64;
+// A pool goes with its context: after cudaDeviceReset the device has another one, of
+// another id, and gets another pool (the old handle is dead and not touched).
+struct Pool {
+  cudaMemPool_t pool = nullptr;
+  unsigned long long context = 0;
+};
 std::mutex g_pool_mutex;
-cudaMemPool_t g_pool[kMaxDevices];
+Pool g_pool[kMaxDevices];
 
+// The id, never used twice in a process, of the context current to this thread.
+// The driver's calls come through the runtime (no libcuda link).
+cudaError_t context_id(unsigned long long* id) {
+  typedef CUresult (*GetCurrent)(CUcontext*);
+  typedef CUresult (*GetId)(CUcontext, unsigned long long*);
+  void *current = nullptr, *get_id = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  cudaError_t e = cudaGetDriverEntryPoint("cuCtxGetCurrent", &current, cudaEnableDefault, &q);
+  if (e == cudaSuccess) e = cudaGetDriverEntryPoint("cuCtxGetId", &get_id, cudaEnableDefault, &q);
+  if (e != cudaSuccess) return e;
+  CUcontext c = nullptr;
+  if (!current || !get_id || reinterpret_cast<GetCurrent>(current)(&c) != CUDA_SUCCESS ||
+      reinterpret_cast<GetId>(get_id)(c, id) != CUDA_SUCCESS)
+    return cudaErrorInitializationError;
+  return cudaSuccess;
+}
+
+// The pool of `device`, which is current.
 cudaError_t pool_of(int device, cudaMemPool_t* pool) {
   if (device >= kMaxDevices) return cudaErrorInvalidDevice;
+  unsigned long long id = 0;
+  const cudaError_t e0 = context_id(&id);
+  if (e0 != cudaSuccess) return e0;
   std::lock_guard<std::mutex> lock(g_pool_mutex);
-  if (!g_pool[device]) {
+  if (!g_pool[device].pool || g_pool[device].context != id) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -249,9 +277,9 @@ cudaError_t pool_of(int device, cudaMemPool_t* pool) {
       cudaMemPoolDestroy(p);
       return e;
     }
-    g_pool[device] = p;
+    g_pool[device] = {p, id};
   }
-  *pool = g_pool[device];
+  *pool = g_pool[device].pool;
   return cudaSuccess;
 }
 
