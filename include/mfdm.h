@@ -406,7 +406,9 @@ int mfdm_dispersion_velocities(double c_min, double c_max, double dc);
  * selected); offsets: host [ntr] signed source-receiver offsets (m); fs:
  * sampling rate (Hz); amplitude: host [nt/2+1][nv] with nv from
  * mfdm_dispersion_velocities. Its device buffers on `device` come from a memory
- * pool of the library, which keeps at most 64 MiB of them between calls. */
+ * pool of the library, which keeps at most 64 MiB of them between calls and gives
+ * those up to the library's other allocations where they would not fit. May be
+ * called from several threads. */
 int mfdm_dispersion_image(const float* gather, int nt, int ntr, const double* offsets, double fs,
                           double c_min, double c_max, double dc, float* amplitude, int device);
 

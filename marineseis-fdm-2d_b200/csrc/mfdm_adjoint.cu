@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "mfdm_adjoint.h"
+#include "mfdm_kernels.h"
 
 namespace mfdm {
 namespace adj {
@@ -962,7 +963,7 @@ cudaError_t scan(const unsigned long long* count, long long* rowptr, long long l
   if (need > *tmp_bytes) {
     if (*tmp) cudaFree(*tmp);
     *tmp = nullptr;
-    if ((e = cudaMalloc(tmp, need)) != cudaSuccess) return e;
+    if ((e = mfdm::device_malloc(tmp, need)) != cudaSuccess) return e;
     *tmp_bytes = need;
   }
   return cub::DeviceScan::ExclusiveSum(*tmp, need, count, out, len + 1, st);
@@ -980,14 +981,14 @@ cudaError_t drop_interior(const CsrT& full, const SetLayout& L, CsrT* rest,
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(count + L.len, 0, sizeof(unsigned long long), st)) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&rest->rowptr, size_t(L.len + 1) * sizeof(long long))) != cudaSuccess) return e;
+  if ((e = mfdm::device_malloc(&rest->rowptr, size_t(L.len + 1) * sizeof(long long))) != cudaSuccess) return e;
   if ((e = scan(count, rest->rowptr, L.len, tmp, tmp_bytes, st)) != cudaSuccess) return e;
   if ((e = cudaMemcpyAsync(&rest->nnz, rest->rowptr + L.len, sizeof(long long),
                            cudaMemcpyDeviceToHost, st)) != cudaSuccess)
     return e;
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&rest->col, size_t(std::max<long long>(rest->nnz, 1)) * sizeof(int))) != cudaSuccess) return e;
-  if ((e = cudaMalloc(&rest->val, size_t(std::max<long long>(rest->nnz, 1)) * sizeof(float))) != cudaSuccess) return e;
+  if ((e = mfdm::device_malloc(&rest->col, size_t(std::max<long long>(rest->nnz, 1)) * sizeof(int))) != cudaSuccess) return e;
+  if ((e = mfdm::device_malloc(&rest->val, size_t(std::max<long long>(rest->nnz, 1)) * sizeof(float))) != cudaSuccess) return e;
   k_drop_fill<<<g, kBlock, 0, st>>>(full.rowptr, full.col, full.val, L, rest->rowptr, rest->col, rest->val);
   return cudaGetLastError();
 }
@@ -1000,17 +1001,17 @@ cudaError_t list_rows(HybridT* H, const SetLayout& L, unsigned long long* flag, 
   if (e != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(flag + L.len, 0, sizeof(unsigned long long), st)) != cudaSuccess) return e;
   long long* pos = nullptr;
-  if ((e = cudaMalloc(&pos, size_t(L.len + 1) * sizeof(long long))) != cudaSuccess) return e;
+  if ((e = mfdm::device_malloc(&pos, size_t(L.len + 1) * sizeof(long long))) != cudaSuccess) return e;
   e = scan(flag, pos, L.len, tmp, tmp_bytes, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&H->nrows, pos + L.len, sizeof(long long), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e == cudaSuccess) e = cudaMalloc(&H->nzrow, size_t(std::max<long long>(H->nrows, 1)) * sizeof(int));
+  if (e == cudaSuccess) e = mfdm::device_malloc(&H->nzrow, size_t(std::max<long long>(H->nrows, 1)) * sizeof(int));
   if (e == cudaSuccess) {
     k_list_rows<<<g, kBlock, 0, st>>>(H->rest.rowptr, pos, L.len, H->nzrow);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMalloc(&H->t, size_t(L.len) * sizeof(float));
+  if (e == cudaSuccess) e = mfdm::device_malloc(&H->t, size_t(L.len) * sizeof(float));
   if (e == cudaSuccess) e = cudaMemsetAsync(H->t, 0, size_t(L.len) * sizeof(float), st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(pos);

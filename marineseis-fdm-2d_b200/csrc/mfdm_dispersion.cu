@@ -226,9 +226,12 @@ __global__ void __launch_bounds__(kIJ * kIS) image_kernel(const double2* __restr
 int err(int code, const char* msg) { return mfdm::set_error(code, msg); }
 
 // Device buffers come from a pool of each device that keeps up to kPoolKeep bytes
-// between calls (the driver takes them back when an allocation would fail):
-// cudaMalloc and cudaFree of one call's 12 MB took 0.6 ms, on a busy host several,
-// against 0.45 ms of kernels. Pools are safe to use from several threads.
+// between calls: cudaMalloc and cudaFree of one call's 12 MB took 0.6 ms, on a busy
+// host several, against 0.45 ms of kernels (the call 1.5 ms with them, 0.84 without).
+// What is above that goes back before the call returns, and the rest when an
+// allocation of this library would fail otherwise (device_malloc): the driver does
+// not take a pool's idle memory for another allocation by itself. Pools are safe to
+// use from several threads.
 constexpr unsigned long long kPoolKeep = 64ull << 20;
 constexpr int kMaxDevices = 64;
 // A pool goes with its context: after cudaDeviceReset the device has another one, of
@@ -283,14 +286,44 @@ cudaError_t pool_of(int device, cudaMemPool_t* pool) {
   return cudaSuccess;
 }
 
+// Gives the pool's idle memory back to the driver but for `keep` bytes, once the
+// frees queued on the default stream have run.
+void trim(cudaMemPool_t pool, unsigned long long keep) {
+  unsigned long long reserved = 0;
+  if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+      reserved > keep && cudaStreamSynchronize(nullptr) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, keep);
+}
+
 struct DevBuf {
+  cudaMemPool_t pool = nullptr;
   void* p = nullptr;
   ~DevBuf() {
-    if (p) cudaFreeAsync(p, nullptr);
+    if (!p) return;
+    cudaFreeAsync(p, nullptr);
+    trim(pool, kPoolKeep);  // every call, so that the last of several at once does
   }
 };
 
 }  // namespace
+
+namespace mfdm {
+cudaError_t device_malloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  int device = 0;
+  unsigned long long id = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device >= kMaxDevices || context_id(&id) != cudaSuccess)
+    return e;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (!g_pool[device].pool || g_pool[device].context != id) return e;
+    trim(g_pool[device].pool, 0);
+  }
+  (void)cudaGetLastError();
+  return cudaMalloc(p, bytes);
+}
+}  // namespace mfdm
 
 extern "C" int mfdm_dispersion_velocities(double c_min, double c_max, double dc) {
   if (!(c_min > 0.0) || !(c_max >= c_min) || !(dc > 0.0) || !std::isfinite(c_max)) return 0;
@@ -328,10 +361,15 @@ extern "C" int mfdm_dispersion_image(const float* gather, int nt, int ntr, const
                xb = size_t(ntr) * sizeof(double), pb = size_t(nf) * ntr * sizeof(double2),
                ab = size_t(nf) * nc * sizeof(float);
   DevBuf d;
-  cudaMemPool_t pool = nullptr;
-  if ((e = pool_of(device, &pool)) != cudaSuccess) return err(MFDM_ERR_CUDA, cudaGetErrorString(e));
-  if ((e = cudaMallocFromPoolAsync(&d.p, up(gb) + up(xb) + up(rb) + up(pb) + ab, pool, nullptr)) !=
-      cudaSuccess) {
+  if ((e = pool_of(device, &d.pool)) != cudaSuccess) return err(MFDM_ERR_CUDA, cudaGetErrorString(e));
+  const size_t bytes = up(gb) + up(xb) + up(rb) + up(pb) + ab;
+  e = cudaMallocFromPoolAsync(&d.p, bytes, d.pool, nullptr);
+  if (e == cudaErrorMemoryAllocation) {  // not while idle blocks of other sizes stay reserved
+    (void)cudaGetLastError();
+    trim(d.pool, 0);
+    e = cudaMallocFromPoolAsync(&d.p, bytes, d.pool, nullptr);
+  }
+  if (e != cudaSuccess) {
     (void)cudaGetLastError();
     return err(MFDM_ERR_NOMEM, cudaGetErrorString(e));
   }

@@ -358,7 +358,7 @@ int ensure_capacity(mfdm_model* m, int steps) {
     for (int b = 0; b < m->nshots; ++b)
       fill_src_table(m->cfg, m->shots[size_t(b)].fpeak, cap, amp.data() + size_t(b) * cap * 4);
     float* d = nullptr;
-    MFDM_CU(cudaMalloc(&d, amp.size() * sizeof(float)));
+    MFDM_CU(mfdm::device_malloc(&d, amp.size() * sizeof(float)));
     MFDM_CU(cudaMemcpy(d, amp.data(), amp.size() * sizeof(float), cudaMemcpyHostToDevice));
     if (m->d_src) cudaFree(m->d_src);
     m->d_src = d;
@@ -371,7 +371,7 @@ int ensure_capacity(mfdm_model* m, int steps) {
     const int cap = std::max(need, m->rec_cap * 2);
     const size_t row = size_t(3) * m->cfg.nx * sizeof(float);  // [shot][sample][3][nx]
     float* d = nullptr;
-    MFDM_CU(cudaMalloc(&d, size_t(m->nshots) * cap * row));
+    MFDM_CU(mfdm::device_malloc(&d, size_t(m->nshots) * cap * row));
     MFDM_CU(cudaMemsetAsync(d, 0, size_t(m->nshots) * cap * row, m->stream));
     if (m->d_rec) {
       MFDM_CU(cudaMemcpy2DAsync(d, size_t(cap) * row, m->d_rec, size_t(m->rec_cap) * row,
@@ -623,7 +623,7 @@ int build(mfdm_model* m, HostModel&& h, int device, const std::vector<ShotCfg>* 
   m->region = roff;
   off = shared + roff * size_t(m->nshots);
   m->dbytes = off;
-  MFDM_CU(cudaMalloc(&m->dmem, off));
+  MFDM_CU(mfdm::device_malloc(&m->dmem, off));
   MFDM_CU(cudaMemsetAsync(m->dmem, 0, off, m->stream));
   char* base = m->dmem;
   auto F = [&](size_t o) { return reinterpret_cast<float*>(base + o); };
@@ -1409,7 +1409,7 @@ Fields fields_at(const mfdm::SetLayout& L, float* base) {
 
 template <class T>
 int dalloc(T** p, size_t n) {
-  MFDM_CU(cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(n, 1) * sizeof(T)));
+  MFDM_CU(mfdm::device_malloc(p, std::max<size_t>(n, 1) * sizeof(T)));
   return MFDM_OK;
 }
 
@@ -1824,7 +1824,7 @@ int mfdm_adjoint_backward(mfdm_model* m, const float* res_svx, const float* res_
   MFDM_CU(cudaStreamWaitEvent(hi, a->ev_enter, 0));
   bool dbl = inner == every && a->nkeep < ncp - 1;
   if (dbl && a->seg2 == nullptr) {
-    if (cudaMalloc(&a->seg2, a->seg_steps * 4 * len * sizeof(float)) != cudaSuccess) {
+    if (mfdm::device_malloc(&a->seg2, a->seg_steps * 4 * len * sizeof(float)) != cudaSuccess) {
       (void)cudaGetLastError();  // not enough memory for two: one buffer, no overlap
       a->seg2 = nullptr;
       dbl = false;
@@ -2040,7 +2040,7 @@ int solid_capacity(mfdm_solid* m, int steps) {
     std::vector<float> amp(size_t(cap) * 4);
     fill_src_table(m->pml, m->fpeak, cap, amp.data());
     float* d = nullptr;
-    MFDM_CU(cudaMalloc(&d, amp.size() * sizeof(float)));
+    MFDM_CU(mfdm::device_malloc(&d, amp.size() * sizeof(float)));
     MFDM_CU(cudaMemcpy(d, amp.data(), amp.size() * sizeof(float), cudaMemcpyHostToDevice));
     if (m->d_src) cudaFree(m->d_src);
     m->d_src = d;
@@ -2051,7 +2051,7 @@ int solid_capacity(mfdm_solid* m, int steps) {
   if (need > m->rec_cap) {
     const int cap = std::max(need, m->rec_cap * 2);
     float* d = nullptr;
-    MFDM_CU(cudaMalloc(&d, size_t(cap) * m->nx * sizeof(float)));
+    MFDM_CU(mfdm::device_malloc(&d, size_t(cap) * m->nx * sizeof(float)));
     MFDM_CU(cudaMemset(d, 0, size_t(cap) * m->nx * sizeof(float)));
     if (m->d_rec) {
       MFDM_CU(cudaMemcpy(d, m->d_rec, size_t(m->rec_cap) * m->nx * sizeof(float),
@@ -2193,7 +2193,7 @@ int solid_build(mfdm_solid* m, const SolidHost& h, int device) {
   }
   const size_t set_floats = (o_set[1] - o_set[0]) / sizeof(float);
   m->dbytes = off;
-  MFDM_CU(cudaMalloc(&m->dmem, off));
+  MFDM_CU(mfdm::device_malloc(&m->dmem, off));
   MFDM_CU(cudaMemsetAsync(m->dmem, 0, off, m->stream));
   char* base = m->dmem;
   auto F = [&](size_t o) { return reinterpret_cast<float*>(base + o); };
@@ -2489,7 +2489,7 @@ class SnapshotDrain {
     DeviceGuard g(m->device);
     MFDM_CU(cudaStreamCreateWithFlags(&copy_, cudaStreamNonBlocking));
     for (int s = 0; s < 2; ++s) {
-      MFDM_CU(cudaMalloc(&dev_[s], n * sizeof(float)));
+      MFDM_CU(mfdm::device_malloc(&dev_[s], n * sizeof(float)));
       MFDM_CU(cudaMallocHost(&host_[s], n * sizeof(float)));
       MFDM_CU(cudaEventCreateWithFlags(&staged_[s], cudaEventDisableTiming));
       MFDM_CU(cudaEventCreateWithFlags(&copied_[s], cudaEventDisableTiming));

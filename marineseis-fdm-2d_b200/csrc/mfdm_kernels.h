@@ -28,6 +28,15 @@ int stage_blocks_per_sm(const Coef& C);
 // Rows per interior tile of a stage launch: C.seg, or by size when 0.
 int stage_seg_rows(const Coef& C);
 
+// cudaMalloc for the library's own buffers: an allocation that does not fit is
+// tried again once the idle memory of the dispersion image's pool has gone back
+// (mfdm_dispersion.cu).
+cudaError_t device_malloc(void** p, size_t bytes);
+template <class T>
+cudaError_t device_malloc(T** p, size_t bytes) {
+  return device_malloc(reinterpret_cast<void**>(p), bytes);
+}
+
 // Library-internal host helpers (mfdm_host.cu): record a failure for
 // mfdm_last_error() and return `code`.
 int set_error(int code, const char* msg);
