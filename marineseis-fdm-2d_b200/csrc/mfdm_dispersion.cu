@@ -139,11 +139,15 @@ __global__ void __launch_bounds__(kDThreads) spectrum_kernel(const float* __rest
       if (k0 + a >= nk || r >= ntr) continue;
       const int k = half == 0 ? k0 + a : nt / 2 - (k0 + a);
       if (half == 1 && k == k0 + a) continue;  // k = nt/4 is its own partner
-      // the unpaired samples: t = 0 and, with even nt, t = nt/2
-      double x = re[a][b] + double(__ldg(g + r)), y = im[a][b];
+      // the unpaired samples: t = 0 and, with even nt, t = nt/2. The product with the
+      // sine of the root 1 stays: infinite samples make it NaN, and the trace silent
+      // at that frequency, as at every other t whose root is 1.
+      const double v0 = double(__ldg(g + r));
+      double x = re[a][b] + v0, y = fma(v0, -0.0, im[a][b]);
       if (fold) {
         const double v = double(__ldg(g + size_t(nt / 2) * ntr + r));
         x += k % 2 ? -v : v;
+        if (k % 2 == 0) y = fma(v, -0.0, y);
       }
       const double mag = sqrt(x * x + y * y);
       P[size_t(k) * ntr + r] = mag > 0.0 ? make_double2(x / mag, -y / mag) : make_double2(0.0, 0.0);
