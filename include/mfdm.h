@@ -70,7 +70,7 @@ typedef struct mfdm_info {
   long long cells;                /* nx * (nz_f + nz_s): cells updated per step */
   long long device_bytes;         /* device memory held by the handle */
   int nshots;                     /* shots stepped together (1 unless opened with mfdm_open_batch) */
-  int seg_rows;                   /* rows per interior tile of the stage launches */
+  int seg_rows;                   /* tile height set or chosen (mfdm_set_tile) */
   int blocks_per_sm;              /* stage kernel build in use: 2, 3 or 4 (mfdm_set_blocks_per_sm) */
 } mfdm_info;
 

@@ -1066,7 +1066,7 @@ int mfdm_set_tile(mfdm_model* m, int seg_rows) {
   DeviceGuard g(m->device);
   MFDM_CU(cudaStreamSynchronize(m->stream));
   m->C.seg = seg_rows;
-  release_graph(m);  // the segment height is baked into the captured launches
+  release_graph(m);  // the tile height is baked into the captured launches
   return MFDM_OK;
 }
 
@@ -1074,16 +1074,16 @@ int mfdm_set_tile(mfdm_model* m, int seg_rows) {
 
 namespace {
 
-const int kSegCandidates[] = {8, 12, 16, 24, 32, 48};
+const int kSegCandidates[] = {8, 16, 24, 32, 48};  // tile heights as they run: multiples of 8
 
 std::mutex g_tune_mu;
 // (device, nx, nz_f, nz_s, npd, bdy, nshots) -> (rows, blocks per SM)
 std::map<std::vector<int>, std::pair<int, int>> g_tune;
 
-// Device time of one captured kGraphSteps-step replay with `seg` rows per segment
+// Device time of one captured kGraphSteps-step replay with tiles of `seg` rows
 // and the stage build of `variant` blocks per SM (after one untimed replay that
 // also captures the graph).
-int time_segment_rows(mfdm_model* m, int seg, int variant, float* ms) {
+int time_tile_rows(mfdm_model* m, int seg, int variant, float* ms) {
   m->C.seg = seg;
   m->C.variant = variant;
   release_graph(m);
@@ -1126,9 +1126,8 @@ int mfdm_autotune(mfdm_model* m, int* seg_rows) {
     float best_ms = 0.f;
     for (int variant = 2; variant <= 4; ++variant)
       for (int i = 0; i < n; ++i) {
-        if (variant == 4 && kSegCandidates[i] % 8 != 0) continue;  // whole multiples of the tile's row step
         float ms = 0.f;
-        if ((rc = time_segment_rows(m, kSegCandidates[i], variant, &ms)) != MFDM_OK) return rc;
+        if ((rc = time_tile_rows(m, kSegCandidates[i], variant, &ms)) != MFDM_OK) return rc;
         if (best.first == 0 || ms < best_ms) {
           best = {kSegCandidates[i], variant};
           best_ms = ms;
@@ -1427,7 +1426,7 @@ int adjoint_build(mfdm_model* m) {
   Coef C = m->C;
   C.srcx = -1;  // the operator without the source
   C.src_pos = nullptr;
-  const int stage = 2;  // the third stage: out = U^n + c k, with U^n = 0, and no accumulator
+  const int stage = 2;  // the third stage: out = U^n + c k, with U^n = 0 (what it adds to the accumulator is not read)
   const float cc = C.rk_c[stage], scale = 1.0f / cc;
   const Fields &Out = m->S[0], &In = m->S[1], &Un = m->S[2], &Acc = m->S[3];
   // cells a stage updates: with input 0 and U^n = 1 the output is 1 exactly there
