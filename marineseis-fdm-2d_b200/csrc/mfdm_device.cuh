@@ -632,26 +632,4 @@ __device__ __forceinline__ float rk_last(float k, float y, float acc, float c) {
   return __fadd_rn(s, fmaf(c, k, e));
 }
 
-// One value updated once a step (the solid-only kernels):
-//   first:  out = y + c k
-//   second: out = Un + c k,  acc = rk_acc
-//   third:  out = Un + c k
-//   last:   out = rk_last
-template <int KIND>
-__device__ __forceinline__ void rk_update(float k, float y, const float* __restrict__ Un,
-                                          float* __restrict__ out, float* __restrict__ acc,
-                                          size_t i, float c, float w) {
-  if (KIND == kStageFirst) {
-    out[i] = fmaf(c, k, y);
-  } else if (KIND == kStageSecond) {
-    const float u = Un[i];
-    out[i] = fmaf(c, k, u);
-    acc[i] = rk_acc(k, y, u, w);
-  } else if (KIND == kStageThird) {
-    out[i] = fmaf(c, k, Un[i]);
-  } else {
-    out[i] = rk_last(k, y, acc[i], c);
-  }
-}
-
 }  // namespace mfdm

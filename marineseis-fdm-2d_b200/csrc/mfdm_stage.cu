@@ -40,8 +40,8 @@ using namespace tiles;
 
 constexpr bool kOnce = MFDM_STAGE_ONCE;
 // Launches of the other builds may start as the stage launch before them ends: the
-// gap between dependent launches is a fifth of a small grid's stage (us a step,
-// plain / chained: 160x121 24.6 / 21.1, 400x400 30.1 / 28.0, 800x400 36.0 / 31.8,
+// gap between dependent launches is 3 to 14 % of a step (us a step, plain /
+// chained: 160x121 24.6 / 21.1, 400x400 30.1 / 28.0, 800x400 36.0 / 31.8,
 // 1200x800 83.8 / 79.7, 2048x1024 177 / 172). A block lets the next grid start once
 // its own operands have arrived, not at its start: the waiting blocks of two later
 // grids would take the slots (160x121 26.4, 800x400 at 16 rows 32.0). Large grids gain nothing
@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(kThreads, MFDM_STAGE_BLOCKS)
   }
 }
 
-// Rows of an interior tile: the segment height rounded up to a multiple of 8, at most 48.
+// Rows of an interior tile: the height set or chosen, rounded up to a multiple of 8, at most 48.
 int tile_rows_of(const Coef& C) {
   const int tr = (stage_seg_rows(C) + kRowStep - 1) / kRowStep * kRowStep;
   return tr < kTileRowsMax ? tr : kTileRowsMax;
