@@ -14,11 +14,12 @@ value  = cells x steps / device time (CUDA events on the solver's stream, max
 e2e    = the same metric through the public API with host buffers: model
          upload from pinned host memory, the steps, and the receiver read-back
          (after one untimed upload), with the three parts' times.
-roofline: algorithmic bytes per step (16 S + 4 M floats per cell: 464 B solid,
-         288 B fluid, +256 B per PML strip cell and direction) over the summed
-         average durations of the four stage launches (filter_launch_ms: what the
-         events see after the last one). The bytes are the reference scheme's; from
-         2.5 million cells the step accumulates once and moves 384 / 240 B a cell.
+roofline: the bytes a step moves (step_bytes; at 4096 x 2048, which accumulates
+         once a step, 12 S + 4 M floats per cell: 384 B solid, 240 B fluid,
+         +192 B per PML strip cell and direction) over the summed average
+         durations of the four stage launches (filter_launch_ms: what the events
+         see after the last one). reference_scheme_bytes_per_step: the bytes of
+         the reference's scheme, 16 S + 4 M floats.
 With N > 1 every rank runs its own copy of the workload (independent shots):
 weak scaling, no data-path collective.
 other_workloads.reference_cuda_build: the reference's own CUDA build
@@ -151,7 +152,8 @@ def reference_cuda_build(workloads, repeats: int = 3) -> dict:
 
 
 def algorithmic_bytes(m) -> int:
-    """Bytes per step a classical-RK4 sweep must move (16 S + 4 M floats per cell)."""
+    """Bytes per step of the reference's scheme, which adds to the accumulator in
+    every stage (16 S + 4 M floats per cell)."""
     fluid = m.nx * m.nz_f * (16 * 3 + 4 * 6) * 4
     solid = m.nx * m.nz_s * (16 * 5 + 4 * 9) * 4
     strips = 2 * m.npd * (m.nz_f - 3) + 2 * m.npd * (m.nz_s - 3) + m.npd * (m.nx - 6)
@@ -161,11 +163,33 @@ def algorithmic_bytes(m) -> int:
 def batched_bytes(m, nshots: int) -> int:
     """Bytes per step of `nshots` shots of one model when the coefficients are
     read once for all shots (each shot still moves its own 16 state floats per
-    field and cell and its ADE memory)."""
+    field and cell and its ADE memory), in the reference's scheme."""
     state = m.nx * m.nz_f * 16 * 3 + m.nx * m.nz_s * 16 * 5
     strips = 2 * m.npd * (m.nz_f - 3) + 2 * m.npd * (m.nz_s - 3) + m.npd * (m.nx - 6)
     coef = m.nx * m.nz_f * 4 * 6 + m.nx * m.nz_s * 4 * 9
     return (nshots * (state + strips * 16 * 4) + coef) * 4
+
+
+ONCE_CELLS = 2_500_000  # from this grid the default build accumulates once a step
+
+
+def step_bytes(m, nshots: int = 1, build: int = 4) -> int:
+    """Bytes per step that the stage kernels of `build` (mfdm_info.blocks_per_sm)
+    move, the coefficients read once for all shots of a batch: batched_bytes with
+    16 floats per state value where every stage adds to the accumulator, and 12
+    where one stage a step does (stage 1: input, output; 2: input, U^n, output,
+    accumulator; 3: input, U^n, output; 4: input, accumulator, output)."""
+    if build != 4 or m.nx * (m.nz_f + m.nz_s) < ONCE_CELLS:
+        return batched_bytes(m, nshots)
+    state = m.nx * m.nz_f * 3 + m.nx * m.nz_s * 5
+    strips = 2 * m.npd * (m.nz_f - 3) + 2 * m.npd * (m.nz_s - 3) + m.npd * (m.nx - 6)
+    return batched_bytes(m, nshots) - nshots * (state + strips * 4) * 4 * 4
+
+
+def solid_step_bytes(m) -> int:
+    """The same for solid only, which accumulates once a step at every size:
+    5 x 12 state floats and 4 x 9 coefficient floats a cell."""
+    return m.cells * (5 * 12 + 4 * 9) * 4
 
 
 def peaks():
@@ -326,12 +350,13 @@ def batched_shots(model, n: int, seed: int = 2):
 def batched_rate(mfdm, model, device: int, warmup: int, nshots: int = 64, steps: int = 300):
     """Shot-steps/s of one batch (one launch per RK stage for all shots) against
     the same shots run one after another through single-shot handles, device
-    time (CUDA events) over `steps` steps each. Both arms pick their segment
-    height with the autotuner first."""
+    time (CUDA events) over `steps` steps each. Both arms pick their tile height
+    and build with the autotuner first."""
     import copy
     shots = batched_shots(model, nshots)
     with mfdm.Batch.from_model(model, shots, device=device) as b:
         tile_b = b.autotune()
+        build = b.info()["blocks_per_sm"]
         b.step(warmup)
         tb, _ = b.time_steps(steps)
     loop_ms = 0.0
@@ -347,15 +372,15 @@ def batched_rate(mfdm, model, device: int, warmup: int, nshots: int = 64, steps:
             loop_ms += t1
     cells = model.cells * nshots * steps
     peak, _ = peaks()
-    shared = batched_bytes(model, nshots) * steps / (tb / 1e3) / 1e9
-    unshared = algorithmic_bytes(model) * nshots * steps / (tb / 1e3) / 1e9
+    shared = step_bytes(model, nshots, build) * steps / (tb / 1e3) / 1e9
+    unshared = step_bytes(model, 1, build) * nshots * steps / (tb / 1e3) / 1e9
     return {"shots": nshots, "steps": steps, "ricker_hz": "U[10, 25], seed 2",
             "value": round(cells / (tb / 1e3) / 1e9, 3), "unit": "Gcell/s",
             "shot_steps_per_s": round(nshots * steps / (tb / 1e3), 1),
             "per_shot_loop_gcells": round(cells / (loop_ms / 1e3) / 1e9, 3),
             "speedup_vs_per_shot_loop": round(loop_ms / tb, 3),
             "seg_rows": {"batch": tile_b, "per_shot": tile_1},
-            "roofline": {"bytes": "coefficients read once per segment for all shots",
+            "roofline": {"bytes": "coefficients read once per tile for all shots",
                          "achieved_gbs": round(shared, 1), "frac": round(shared / peak, 4),
                          "frac_if_unshared": round(unshared / peak, 4)}}
 
@@ -365,11 +390,12 @@ def uneven_rate(mfdm, device: int, nmodels: int = 32, steps: int = 128):
     400..2000, nz 300..1000, seed 3) stepped together as one group (one
     captured graph, the models on parallel branches) against the same models
     stepped one after another, each through its own captured graph. Every model
-    gets its segment height from the autotuner first; device time (CUDA events)."""
+    gets its tile height and build from the autotuner first; device time (CUDA events)."""
     models = modelgen.uneven_models(nmodels, seed=3, nt=10)
     solvers = [mfdm.Solver.from_model(m, device=device) for m in models]
     try:
         tiles = [s.autotune() for s in solvers]
+        builds = [s.info()["blocks_per_sm"] for s in solvers]
         loop_ms = 0.0
         for s in solvers:
             s.set_shot(0, reset=True)
@@ -386,7 +412,7 @@ def uneven_rate(mfdm, device: int, nmodels: int = 32, steps: int = 128):
             s.close()
     cells = sum(m.cells for m in models) * steps
     peak, _ = peaks()
-    gbs = sum(algorithmic_bytes(m) for m in models) * steps / (tg / 1e3) / 1e9
+    gbs = sum(step_bytes(m, 1, b) for m, b in zip(models, builds)) * steps / (tg / 1e3) / 1e9
     return {"models": nmodels, "steps": steps, "cells": sum(m.cells for m in models),
             "value": round(cells / (tg / 1e3) / 1e9, 3), "unit": "Gcell/s",
             "model_loop_gcells": round(cells / (loop_ms / 1e3) / 1e9, 3),
@@ -567,8 +593,8 @@ def large_adjoint_rate(mfdm, device: int, nshots: int = 1, nsteps: int = 200, ev
 def solid_only_rate(mfdm, device: int, n: int = 2048, steps: int = 256):
     """Solid only with a free surface (calc_type 0) on an n x n grid with surface
     topography: device time of `steps` graph-captured steps, and the whole
-    step's share of the HBM roofline at the solid's algorithmic 464 B per
-    cell-step (16 state + 4 x 9 coefficient floats x 4 B)."""
+    step's share of the HBM roofline at the 384 B per cell-step it moves
+    (solid_step_bytes)."""
     m = modelgen.make_solid_model(n, n, npd=20, fpeak=15.0, dt=5e-4, nt=10, src_x=[n // 2],
                                   src_z=[20], amp=20.0, wavelength=600.0)
     with mfdm.SolidSolver.from_model(m, device=device) as s:
@@ -586,7 +612,7 @@ def solid_only_rate(mfdm, device: int, n: int = 2048, steps: int = 256):
     errs = {k: rel_l2(a, b) for k, a, b in zip(names, ours, ref["solid"])}
     worst = max(errs, key=errs.get)
     gcells = m.cells * steps / (ms / 1e3) / 1e9
-    gbs = m.cells * 464 * steps / (ms / 1e3) / 1e9
+    gbs = solid_step_bytes(m) * steps / (ms / 1e3) / 1e9
     peak, _ = peaks()
     return {"grid": f"{n}x{n}", "steps": steps, "value": round(gcells, 3), "unit": "Gcell/s",
             "ms_per_step": round(ms / steps, 4), "achieved_gbs": round(gbs, 1),
@@ -607,7 +633,7 @@ def main():
     ap.add_argument("--blocks-per-sm", type=int, default=0, choices=[0, 2, 3, 4],
                     help="stage kernel build (0: the default, as for any model)")
     ap.add_argument("--seg-rows", type=int, default=0,
-                    help="rows per segment block of the stage launches (0: the default for the grid)")
+                    help="rows per interior tile of the stage launches (0: the default for the grid)")
     ap.add_argument("--adjoint-profile", action="store_true",
                     help="only a short adjoint run on a curvilinear model (16 steps, checkpoint "
                          "every 8, seeded residuals): a launch list of the adjoint kernels for ncu")
@@ -669,6 +695,7 @@ def main():
     solver = mfdm.Solver.from_model(model, device=local)
     solver.set_blocks_per_sm(args.blocks_per_sm)
     solver.set_tile(args.seg_rows)
+    build = solver.info()["blocks_per_sm"]
     solver.set_shot(0, reset=True)
     solver.step(args.warmup)
 
@@ -693,7 +720,7 @@ def main():
     nk = min(args.steps, 200)
     _, kms = solver.time_steps(nk, per_kernel=True)
     stage_ms = sum(kms[:4]) / nk  # the four stage launches of one step
-    alg = algorithmic_bytes(model)
+    alg = step_bytes(model, 1, build)
     peak, peak_kind = peaks()
     achieved = alg / (stage_ms / 1e3) / 1e9
     traffic = None
@@ -761,8 +788,9 @@ def main():
         other["batched_1200x800_64_shots"] = batched_rate(mfdm, small, local, args.warmup)
         other["batched_1200x800_64_shots"]["fp64_error"] = dict(
             fp64_error(mfdm, small, 300, local, shot=batched_shots(small, 64)[0]),
-            note="shot 0 with its own frequency; every batched shot is bit-identical to "
-                 "the same shot run alone (tests/test_gpu_batch.py)")
+            note="shot 0 with its own frequency; with the default build every batched shot is "
+                 "bit-identical to the same shot run alone (tests/test_gpu_batch.py, "
+                 "tests/test_gpu_batch_sizes.py)")
         other["uneven_32_models"] = uneven_rate(mfdm, local)
         m0 = modelgen.uneven_models(1, seed=3, nt=10)[0]
         other["uneven_32_models"]["fp64_error"] = dict(
@@ -807,6 +835,7 @@ def main():
                          "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": traffic,
                          "peak_kind": peak_kind,
                          "algorithmic_bytes_per_step": alg,
+                         "reference_scheme_bytes_per_step": algorithmic_bytes(model),
                          "stage_launch_ms": [round(k / nk, 5) for k in kms[:4]],
                          "filter_launch_ms": round(kms[4] / nk, 5)},
             "gpu_launches": 4 * args.steps,
