@@ -188,8 +188,7 @@ int mfdm_batch_get_field(mfdm_model* m, int shot, int field, float* host);
 /* Sets the tile height: a multiple of 4 in [4, 128] (the kernels round it up
  * to a multiple of 8 and cap it at 48), or 0 for the default (8 rows below 0.2 M
  * cells per launch, counting every shot of a batch, 16 below 0.5 M, 24 below
- * 4 M, 32 above). Results do not depend on it beyond FP32 rounding of the last
- * bit. */
+ * 4 M, 32 above). Results do not depend on it. */
 int mfdm_set_tile(mfdm_model* m, int seg_rows);
 
 /* Selects the stage kernel build by its register budget: 2 or 3 resident blocks
