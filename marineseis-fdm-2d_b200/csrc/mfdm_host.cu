@@ -350,6 +350,10 @@ void release_graph(mfdm_model* m) {
   }
 }
 
+bool fits_capacity(const mfdm_model* m, int steps) {
+  return steps <= m->src_steps && (steps + m->gap - 1) / m->gap <= m->rec_cap;
+}
+
 // Grows the source table and the receiver buffer so that steps up to `steps` fit.
 int ensure_capacity(mfdm_model* m, int steps) {
   if (steps > m->src_steps) {
@@ -929,9 +933,17 @@ int mfdm_update_rk4(mfdm_model* m, int it, void* stream) {
   if (!m) return fail(MFDM_ERR_ARG, "null handle");
   if (it < 0) return fail(MFDM_ERR_ARG, "negative time index");
   DeviceGuard g(m->device);
+  cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : m->stream;
+  if (st != m->stream && !fits_capacity(m, it + 1)) {
+    // the buffers grow on the handle's stream: the samples that steps on the
+    // caller's stream still have to write must be there before they are copied
+    // (a capturing stream has nothing in flight)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    MFDM_CU(cudaStreamIsCapturing(st, &cap));
+    if (cap == cudaStreamCaptureStatusNone) MFDM_CU(cudaStreamSynchronize(st));
+  }
   int rc = ensure_capacity(m, it + 1);
   if (rc != MFDM_OK) return rc;
-  cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : m->stream;
   if (st != m->stream) MFDM_CU(cudaStreamSynchronize(m->stream));
   rc = enqueue_step(m, it, st, nullptr, false, st == m->stream, st == m->stream);  // the caller's stream: plain launches
   if (rc != MFDM_OK) return rc;
