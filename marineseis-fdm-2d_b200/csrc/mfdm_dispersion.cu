@@ -248,18 +248,19 @@ std::mutex g_pool_mutex;
 Pool g_pool[kMaxDevices];
 
 // The id, never used twice in a process, of the context current to this thread.
-// The driver's calls come through the runtime (no libcuda link).
+// The driver's calls come through the runtime (no libcuda link), looked up once.
+void* driver_call(const char* name) {
+  void* p = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  return cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess ? p : nullptr;
+}
 cudaError_t context_id(unsigned long long* id) {
   typedef CUresult (*GetCurrent)(CUcontext*);
   typedef CUresult (*GetId)(CUcontext, unsigned long long*);
-  void *current = nullptr, *get_id = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  cudaError_t e = cudaGetDriverEntryPoint("cuCtxGetCurrent", &current, cudaEnableDefault, &q);
-  if (e == cudaSuccess) e = cudaGetDriverEntryPoint("cuCtxGetId", &get_id, cudaEnableDefault, &q);
-  if (e != cudaSuccess) return e;
+  static const GetCurrent get_current = reinterpret_cast<GetCurrent>(driver_call("cuCtxGetCurrent"));
+  static const GetId get_id = reinterpret_cast<GetId>(driver_call("cuCtxGetId"));
   CUcontext c = nullptr;
-  if (!current || !get_id || reinterpret_cast<GetCurrent>(current)(&c) != CUDA_SUCCESS ||
-      reinterpret_cast<GetId>(get_id)(c, id) != CUDA_SUCCESS)
+  if (!get_current || !get_id || get_current(&c) != CUDA_SUCCESS || get_id(c, id) != CUDA_SUCCESS)
     return cudaErrorInitializationError;
   return cudaSuccess;
 }
